@@ -1,4 +1,4 @@
-// Ion flights: one thread per ion.  Restates Trajectory_3d (tapsim/
+// Ion flights: one warp per ion.  Restates Trajectory_3d (tapsim/
 // trajectory_3d.cpp) in FP64: the embedded Cash-Karp Runge-Kutta step
 // (o5_integrator, :583-676, tableau of Cash & Karp 1990), the
 // error-restricted step control (errorRestricted_stepper, :358-425), the
@@ -10,8 +10,6 @@
 // geometry_3d.cpp:916-980); the tetrahedron comes from a visibility walk
 // (findTetrahedron, geometry_3d.cpp:988-1044) whose start face rotates
 // instead of being drawn with rand().
-#include <algorithm>
-
 #include "kernels.cuh"
 
 namespace tgd {
@@ -214,7 +212,7 @@ __global__ void k_pack_tets(DevMesh m, float* pack) {
 }
 
 __device__ V3 vertex_field(const DevMesh& m, int i) {
-    const V3 E{m.vfield[3 * i], m.vfield[3 * i + 1], m.vfield[3 * i + 2]};
+    const V3 E{m.vfield[3 * (size_t)i], m.vfield[3 * (size_t)i + 1], m.vfield[3 * (size_t)i + 2]};
     if (E.x != E.x) {
         atomicOr(m.status, S_SINGULAR);
         return V3{0, 0, 0};
@@ -222,31 +220,27 @@ __device__ V3 vertex_field(const DevMesh& m, int i) {
     return E;
 }
 
-// The last tetrahedron an ion touched, from its packed record, with the
-// vertex fields once interpolated from: RK stages that stay inside it need
-// no memory traffic.  A record comes in one round trip; the vertex
-// fields of the final tetrahedron of a walk take a second.  Every member is
-// addressed with compile-time indices so that the cache lives in registers.
-struct TetSlot {
+// One lane's slot of the warp's tetrahedra (see trace_ion): a packed record,
+// and the vertex fields once interpolated from.  Every member is addressed
+// with compile-time indices so that the slot lives in registers.  An empty
+// slot has t = -1 and zero gradients, which hold no point.
+struct LaneTet {
     int t;
     int nb0, nb1, nb2, nb3;
     int v0, v1, v2, v3;
+    float vol6;
+    bool hasF;
     V3 P0;
     V3 G1, G2, G3;
-    float vol6;
+    double gmax;  // 3e-13 times the largest gradient component
     V3 F0, F1, F2, F3;
-    bool hasF;
-};
-// `a` is the tetrahedron of the last lookup
-struct TetCache {
-    TetSlot a;
 };
 
 __device__ __forceinline__ int pick4(int k, int x0, int x1, int x2, int x3) {
     return k == 0 ? x0 : (k == 1 ? x1 : (k == 2 ? x2 : x3));
 }
 
-__device__ void load_slot(const DevMesh& m, TetSlot& s, int t) {
+__device__ __forceinline__ void load_slot(const DevMesh& m, LaneTet& s, int t) {
     const float4* p = reinterpret_cast<const float4*>(m.tetpack + kTetWords * (size_t)t);
     const float4 q0 = __ldg(p);
     const double2 g0 = __ldg(reinterpret_cast<const double2*>(p + 1));
@@ -262,6 +256,10 @@ __device__ void load_slot(const DevMesh& m, TetSlot& s, int t) {
     s.G1 = V3{g0.x, g0.y, g1.x};
     s.G2 = V3{g1.y, g2.x, g2.y};
     s.G3 = V3{g3.x, g3.y, g4.x};
+    const double m1 = fmax(fmax(fabs(s.G1.x), fabs(s.G1.y)), fabs(s.G1.z));
+    const double m2 = fmax(fmax(fabs(s.G2.x), fabs(s.G2.y)), fabs(s.G2.z));
+    const double m3 = fmax(fmax(fabs(s.G3.x), fabs(s.G3.y)), fabs(s.G3.z));
+    s.gmax = 3e-13 * fmax(m1, fmax(m2, m3));
     const long long nb01 = __double_as_longlong(g4.y);
     s.nb0 = (int)(unsigned)(nb01 & 0xffffffffll);
     s.nb1 = (int)(unsigned)((unsigned long long)nb01 >> 32);
@@ -274,118 +272,133 @@ __device__ void load_slot(const DevMesh& m, TetSlot& s, int t) {
     s.hasF = false;
 }
 
-// Barycentric coordinates of p in the slot's tetrahedron and bounds on their
-// rounding error (about a thousand ulps of the terms summed)
+// Products and sums unfused, and in lane_field fused in a stated order: the
+// step control's decisions turn on the last digit of the fields, so the
+// arithmetic must not change with what the compiler finds to share.
+__device__ __forceinline__ double dot_rn(V3 g, double x, double y, double z) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(g.x, x), __dmul_rn(g.y, y)), __dmul_rn(g.z, z));
+}
+
+// Barycentric coordinates of p in this lane's tetrahedron.  *inside: p lies
+// inside for certain, every coordinate above a bound that is at least the
+// rounding bounds the walk works with (1e-13 times the absolute sums of the
+// products), so that the walk could end in no other tetrahedron.
 struct Bary {
-    double l0, l1, l2, l3, e0, e1, e2, e3;
+    double l0, l1, l2, l3;
 };
-__device__ __forceinline__ Bary lambdas(const TetSlot& S, V3 p) {
+__device__ __forceinline__ Bary lane_bary(const LaneTet& S, V3 p, bool* inside) {
     const double dx = p.x - S.P0.x, dy = p.y - S.P0.y, dz = p.z - S.P0.z;
     Bary b;
-    b.l1 = S.G1.x * dx + S.G1.y * dy + S.G1.z * dz;
-    b.l2 = S.G2.x * dx + S.G2.y * dy + S.G2.z * dz;
-    b.l3 = S.G3.x * dx + S.G3.y * dy + S.G3.z * dz;
-    const double a1 = fabs(S.G1.x * dx) + fabs(S.G1.y * dy) + fabs(S.G1.z * dz);
-    const double a2 = fabs(S.G2.x * dx) + fabs(S.G2.y * dy) + fabs(S.G2.z * dz);
-    const double a3 = fabs(S.G3.x * dx) + fabs(S.G3.y * dy) + fabs(S.G3.z * dz);
+    b.l1 = dot_rn(S.G1, dx, dy, dz);
+    b.l2 = dot_rn(S.G2, dx, dy, dz);
+    b.l3 = dot_rn(S.G3, dx, dy, dz);
     b.l0 = 1.0 - b.l1 - b.l2 - b.l3;
-    b.e1 = 1e-13 * a1;
-    b.e2 = 1e-13 * a2;
-    b.e3 = 1e-13 * a3;
-    b.e0 = 1e-13 * (1.0 + a1 + a2 + a3);
+    const double thr = S.gmax * (fabs(dx) + fabs(dy) + fabs(dz)) + 1e-13;
+    *inside = b.l0 > thr && b.l1 > thr && b.l2 > thr && b.l3 > thr;
     return b;
 }
 
-// Makes `a` hold tetrahedron t (loading it unless it is already there)
-__device__ __forceinline__ void cache_tet(const DevMesh& m, TetCache& c, int t) {
-    if (c.a.t == t) return;
-    load_slot(m, c.a, t);
-}
-
-// Side of face k (opposite vertex k) that p lies on: -1 beyond it.  The
-// barycentric coordinate decides unless it is within its rounding bound of
-// zero, or the tetrahedron is flat; then the exact predicate on the vertex
-// coordinates decides (as Predicates::orient3d does in the reference).
+// Sign of the side of face k (opposite vertex k) that p lies on, from the
+// exact predicate on the vertex coordinates (as Predicates::orient3d decides
+// in the reference).
 __device__ __noinline__ int face_side_exact(const float* xyz, double snap, int i0, int i1, int i2, V3 p) {
     return orient_sign(ld3(xyz, i0), ld3(xyz, i1), ld3(xyz, i2), p, snap);
 }
-__device__ __forceinline__ bool beyond(const DevMesh& m, const TetSlot& S, int k, V3 p, double lam, double err) {
-    if (S.vol6 != 0.0f) {
-        if (lam < -err) return true;
-        if (lam > err) return false;
+
+// The neighbour through which a walk to p leaves this lane's tetrahedron
+// (-1: the hull), kHere when p lies beyond none of its faces.  The faces are
+// tried in an order rotating from walk step to walk step.  A barycentric
+// coordinate decides its face unless it is within its rounding bound of
+// zero (about a thousand ulps of the terms summed), or the tetrahedron is
+// flat; then the exact predicate decides.
+constexpr int kHere = -3;
+__device__ __forceinline__ int walk_exit(const DevMesh& m, const LaneTet& S, V3 p, const Bary& b, unsigned rot) {
+    const double dx = p.x - S.P0.x, dy = p.y - S.P0.y, dz = p.z - S.P0.z;
+    const double a1 = fabs(S.G1.x * dx) + fabs(S.G1.y * dy) + fabs(S.G1.z * dz);
+    const double a2 = fabs(S.G2.x * dx) + fabs(S.G2.y * dy) + fabs(S.G2.z * dz);
+    const double a3 = fabs(S.G3.x * dx) + fabs(S.G3.y * dy) + fabs(S.G3.z * dz);
+    const double e1 = 1e-13 * a1, e2 = 1e-13 * a2, e3 = 1e-13 * a3, e0 = 1e-13 * (1.0 + a1 + a2 + a3);
+    unsigned out = (b.l0 < -e0 ? 1u : 0u) | (b.l1 < -e1 ? 2u : 0u) | (b.l2 < -e2 ? 4u : 0u) | (b.l3 < -e3 ? 8u : 0u);
+    unsigned sure = out | (b.l0 > e0 ? 1u : 0u) | (b.l1 > e1 ? 2u : 0u) | (b.l2 > e2 ? 4u : 0u) |
+                    (b.l3 > e3 ? 8u : 0u);
+    if (S.vol6 == 0.0f) out = sure = 0u;
+    for (unsigned left = ~sure & 15u; left; left &= left - 1u) {
+        const int k = __ffs((int)left) - 1;
+        const int i0 = pick4(kFaceDev[k][0], S.v0, S.v1, S.v2, S.v3);
+        const int i1 = pick4(kFaceDev[k][1], S.v0, S.v1, S.v2, S.v3);
+        const int i2 = pick4(kFaceDev[k][2], S.v0, S.v1, S.v2, S.v3);
+        if (face_side_exact(m.xyz, m.snap, i0, i1, i2, p) < 0) out |= 1u << k;
     }
-    const int i0 = pick4(kFaceDev[k][0], S.v0, S.v1, S.v2, S.v3);
-    const int i1 = pick4(kFaceDev[k][1], S.v0, S.v1, S.v2, S.v3);
-    const int i2 = pick4(kFaceDev[k][2], S.v0, S.v1, S.v2, S.v3);
-    return face_side_exact(m.xyz, m.snap, i0, i1, i2, p) < 0;
+    if (out == 0u) return kHere;
+    const unsigned r = rot & 3u;
+    const unsigned turned = (out >> r) | (out << (4u - r));  // bit j: face (r + j) & 3
+    const int k = (int)((r + (unsigned)__ffs((int)turned) - 1u) & 3u);
+    return pick4(k, S.nb0, S.nb1, S.nb2, S.nb3);
 }
 
-// findTetrahedron through the cache: on return c.a holds p's tetrahedron
-// (result 0; *found, when given, p's barycentric coordinates in it), or -1
-// when p is outside the mesh, -2 when the walk exceeded its bound.  The faces are tested in an order rotating from walk step to
-// walk step; the walk leaves through the first face p lies beyond.
-__device__ __forceinline__ int locate_cached(const DevMesh& m, TetCache& c, V3 p, int t, int limit, unsigned& rot,
-                                             Bary* found = nullptr) {
-    if (t < 0) return -1;
+// findTetrahedron over the warp's tetrahedra.  On entry S is the lane whose
+// tetrahedron the walk starts from, b every lane's coordinates of p and bo
+// those of a second point (other), which a slot loaded on the way gets as
+// well.  Returns 0 with S the lane holding p's tetrahedron, -1 when p is
+// outside the mesh, -2 when the walk exceeded its bound.  `next` is the slot
+// that the next new record goes to, in turn; the slot `keep` stays.
+__device__ __forceinline__ int warp_walk(const DevMesh& m, LaneTet& T, int lane, int& S, int& next, int keep, V3 p,
+                                         Bary& b, V3 other, Bary& bo, bool& inOther, int limit, unsigned& rot) {
     for (int step = 0; step < limit; step++) {
-        cache_tet(m, c, t);
-        const TetSlot& S = c.a;
-        const Bary b = lambdas(S, p);
-        const int r = (int)(rot++ & 3u);
-        int next = 0;
-        bool moved = false;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int k = (r + j) & 3;
-            if (!moved) {
-                const double lam = k == 0 ? b.l0 : (k == 1 ? b.l1 : (k == 2 ? b.l2 : b.l3));
-                const double err = k == 0 ? b.e0 : (k == 1 ? b.e1 : (k == 2 ? b.e2 : b.e3));
-                if (beyond(m, S, k, p, lam, err)) {
-                    next = pick4(k, S.nb0, S.nb1, S.nb2, S.nb3);
-                    moved = true;
-                }
-            }
-        }
-        if (!moved) {
-            if (found) *found = b;
+        int to = kHere;
+        if (lane == S) to = walk_exit(m, T, p, b, rot);
+        rot++;
+        to = __shfl_sync(0xffffffffu, to, S);
+        if (to == kHere) {
+            // a flat tetrahedron weights its vertices alike
+            if (lane == S && T.vol6 == 0.0f) b.l0 = b.l1 = b.l2 = b.l3 = 0.25;
             return 0;
         }
-        if (next < 0) return -1;
-        t = next;
+        if (to < 0) return -1;
+        const unsigned have = __ballot_sync(0xffffffffu, T.t == to);
+        if (have) {
+            S = __ffs((int)have) - 1;
+            continue;
+        }
+        next = (next + 1) & 31;
+        if (next == keep) next = (next + 1) & 31;
+        if (lane == next) {
+            load_slot(m, T, to);
+            bool in;
+            b = lane_bary(T, p, &in);
+            bo = lane_bary(T, other, &inOther);
+        }
+        S = next;
     }
     return -2;
 }
 
-// Field at p: walk from `guess`, interpolate the vertex fields with the
-// weights |lambda_k| (1/4 each in a flat tetrahedron).  *located is the
-// tetrahedron holding p (unchanged when p is outside the mesh).
-__device__ __forceinline__ bool fast_field(const DevMesh& m, TetCache& c, V3 p, int guess, int limit, unsigned& rot, V3* E,
-                           int* located) {
-    *E = V3{0, 0, 0};
-    Bary b;  // the walk's last coordinates: p's in the tetrahedron it found
-    const int sl = locate_cached(m, c, p, guess, limit, rot, &b);
-    if (sl == -2) return false;
-    if (sl < 0) return true;
-    TetSlot& S = c.a;
-    *located = S.t;
-    if (!S.hasF) {
-        S.F0 = vertex_field(m, S.v0);
-        S.F1 = vertex_field(m, S.v1);
-        S.F2 = vertex_field(m, S.v2);
-        S.F3 = vertex_field(m, S.v3);
-        S.hasF = true;
-    }
-    double w0 = 0.25, w1 = 0.25, w2 = 0.25, w3 = 0.25;
-    if (S.vol6 != 0.0f) {
-        w0 = fabs(b.l0);
-        w1 = fabs(b.l1);
-        w2 = fabs(b.l2);
-        w3 = fabs(b.l3);
-    }
-    E->x = w0 * S.F0.x + w1 * S.F1.x + w2 * S.F2.x + w3 * S.F3.x;
-    E->y = w0 * S.F0.y + w1 * S.F1.y + w2 * S.F2.y + w3 * S.F3.y;
-    E->z = w0 * S.F0.z + w1 * S.F1.z + w2 * S.F2.z + w3 * S.F3.z;
-    return true;
+// The vertex fields of this lane's tetrahedron, once per record
+__device__ __forceinline__ void lane_load_fields(const DevMesh& m, LaneTet& T) {
+    if (T.hasF) return;
+    T.F0 = vertex_field(m, T.v0);
+    T.F1 = vertex_field(m, T.v1);
+    T.F2 = vertex_field(m, T.v2);
+    T.F3 = vertex_field(m, T.v3);
+    T.hasF = true;
+}
+
+__device__ __forceinline__ double weighted(const Bary& b, double f0, double f1, double f2, double f3) {
+    return fma(fabs(b.l3), f3, fma(fabs(b.l2), f2, fma(fabs(b.l0), f0, __dmul_rn(fabs(b.l1), f1))));
+}
+
+// Component c of the field interpolated in lane S's tetrahedron with the
+// weights |b| (FastField::compute).
+__device__ __forceinline__ double lane_field(const LaneTet& T, const Bary& b, int S, int c) {
+    const double x = __shfl_sync(0xffffffffu, weighted(b, T.F0.x, T.F1.x, T.F2.x, T.F3.x), S);
+    const double y = __shfl_sync(0xffffffffu, weighted(b, T.F0.y, T.F1.y, T.F2.y, T.F3.y), S);
+    const double z = __shfl_sync(0xffffffffu, weighted(b, T.F0.z, T.F1.z, T.F2.z, T.F3.z), S);
+    return c == 0 ? x : (c == 1 ? y : z);
+}
+
+// A vector whose component c the lanes with that component hold
+__device__ __forceinline__ V3 gather3(double v) {
+    return V3{__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1), __shfl_sync(0xffffffffu, v, 2)};
 }
 
 __device__ double potential_at(const DevMesh& m, const double* phi, V3 p, int t) {
@@ -416,53 +429,43 @@ __device__ bool boundary_tet(const DevMesh& m, int t) {
 }
 
 // The accept / retry rule of the steppers other than the error-restricted
-// one of the main path: 0 NONE takes every step; 2 geometryRestricted_stepper
+// one of the main path, for a trial point located in tetrahedron nt (< 0:
+// outside the mesh): 0 NONE takes every step; 2 geometryRestricted_stepper
 // (trajectory_3d.cpp:427-452) accepts a point in a tetrahedron sharing a
 // vertex with the current one (or outside the mesh from a boundary
 // tetrahedron), grows dt by 1.1 while the point stays in the current
 // tetrahedron and shrinks it by 0.9 otherwise; 3 adaptive_stepper
 // (:454-532) shrinks dt by 0.1 when the point leaves that set, then applies
-// the error rule.  Returns 1 to accept, 0 to retry with the updated dt; *nt
-// is the located tetrahedron when *located.
-__device__ __forceinline__ int stepper_verdict(const DevMesh& m, TetCache& fc, const TraceParams& tp, V3 nx, int tet,
-                                            int& cur, unsigned& rot, double rel, double* dt, int* nt, bool* located) {
-    *located = false;
-    if (tp.stepper == 0) return 1;
-    if (tp.stepper == 2 || tp.stepper == 3) {
-        const int nsl = locate_cached(m, fc, nx, cur, tp.walk_limit, rot);
-        *nt = nsl >= 0 ? fc.a.t : nsl;
-        if (*nt == -2) atomicOr(m.status, S_WALK_LIMIT);
-        if (*nt >= 0) cur = *nt;
-        *located = true;
-        if (tp.stepper == 2) {
-            if (*nt < 0 && boundary_tet(m, tet)) return 1;
-            if (shares_vertex(m, tet, *nt)) return 1;
-            if (*nt == tet) {
-                *dt *= 1.1;
-            } else {
-                if (*dt == tp.dt_min) return 1;
-                *dt *= 0.9;
-            }
-            *located = false;
-            return 0;
+// the error rule.  Returns true to accept, false to retry with the updated
+// dt.
+__device__ __forceinline__ bool stepper_verdict(const DevMesh& m, const TraceParams& tp, int tet, int nt, double rel,
+                                                double* dt) {
+    if (tp.stepper == 0) return true;
+    if (tp.stepper == 2) {
+        if (nt < 0 && boundary_tet(m, tet)) return true;
+        if (shares_vertex(m, tet, nt)) return true;
+        if (nt == tet) {
+            *dt *= 1.1;
+        } else {
+            if (*dt == tp.dt_min) return true;
+            *dt *= 0.9;
         }
-        if (*nt >= 0 && *nt != tet && !shares_vertex(m, tet, *nt)) {
-            *dt *= 0.1;
-            *located = false;
-            return 0;
-        }
+        return false;
+    }
+    if (tp.stepper == 3 && nt >= 0 && nt != tet && !shares_vertex(m, tet, nt)) {
+        *dt *= 0.1;
+        return false;
     }
     if (rel < tp.tol || *dt == tp.dt_min) {
         if (rel != 0.0) {
             const double tmp = *dt * pow(tp.tol / rel, 0.25) * 0.9;
             if (tmp < *dt) *dt *= 1.1; else *dt = tmp;
         }
-        return 1;
+        return true;
     }
     const double tmp = *dt * pow(tp.tol / rel, 0.25) * 0.9;
     if (tmp > *dt) *dt *= 0.9; else *dt = tmp;
-    *located = false;
-    return 0;
+    return false;
 }
 
 // Point idx of the path of ion `slot` (Trajectory_3d::phaseVector,
@@ -474,23 +477,42 @@ __device__ __forceinline__ void path_point(const TraceParams& tp, int slot, int 
     p[1] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(tet < 0 ? -1 : tet));
 }
 
-// The error vector of the latest trial step, parked in words 6..11 of the
-// ion's error record so that it holds no registers across the stepper's
-// point location.
-__device__ __forceinline__ void path_trial_error(const TraceParams& tp, int slot, V3 ex, V3 ev) {
-    float* e = tp.path_err + 12 * (size_t)slot + 6;
-    e[0] = (float)ex.x; e[1] = (float)ex.y; e[2] = (float)ex.z;
-    e[3] = (float)ev.x; e[4] = (float)ev.y; e[5] = (float)ev.z;
+// The Cash-Karp tableau (Cash & Karp 1990) by rounds of two stages (see
+// ck_trial): for the stages a = 2r and b = 2r + 1 of round r, the weight of
+// a in b, those of a and of b in the next four stages (0 past the sixth),
+// the fifth-order weights of a and b, and their differences to the
+// fourth-order ones.
+constexpr double kC5[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0, 0.0, 512.0 / 1771.0};
+constexpr double kC4[6] = {2825.0 / 27648.0, 0.0, 18575.0 / 48384.0, 13525.0 / 55296.0, 277.0 / 14336.0, 1.0 / 4.0};
+constexpr double kB20 = 3.0 / 40.0, kB21 = 9.0 / 40.0, kB30 = 3.0 / 10.0, kB31 = -9.0 / 10.0, kB32 = 6.0 / 5.0,
+                 kB40 = -11.0 / 54.0, kB41 = 5.0 / 2.0, kB42 = -70.0 / 27.0, kB43 = 35.0 / 27.0,
+                 kB50 = 1631.0 / 55296.0, kB51 = 175.0 / 512.0, kB52 = 575.0 / 13824.0, kB53 = 44275.0 / 110592.0,
+                 kB54 = 253.0 / 4096.0;
+#define TG_CK_ROUNDS(R)                                                                                            \
+    {{(R)(1.0 / 5.0), (R)kB20, (R)kB30, (R)kB40, (R)kB50, (R)kB21, (R)kB31, (R)kB41, (R)kB51, (R)kC5[0],           \
+      (R)kC5[1], (R)(kC5[0] - kC4[0]), (R)(kC5[1] - kC4[1])},                                                      \
+     {(R)kB32, (R)kB42, (R)kB52, (R)0, (R)0, (R)kB43, (R)kB53, (R)0, (R)0, (R)kC5[2], (R)kC5[3],                   \
+      (R)(kC5[2] - kC4[2]), (R)(kC5[3] - kC4[3])},                                                                 \
+     {(R)kB54, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)kC5[4], (R)kC5[5], (R)(kC5[4] - kC4[4]),         \
+      (R)(kC5[5] - kC4[5])}}
+__constant__ double kCk64[3][13] = TG_CK_ROUNDS(double);
+__constant__ float kCk32[3][13] = TG_CK_ROUNDS(float);
+template <typename R>
+__device__ __forceinline__ R ck_coef(int r, int i) {
+    if constexpr (sizeof(R) == 8) return kCk64[r][i];
+    else return kCk32[r][i];
 }
 
-// Trajectory_3d::cumulative_error (trajectory_3d.cpp:683-700) with the
-// accepted step's error: each of the six components becomes
-// sqrt(current^2 + step^2), in float as the reference keeps it.
-__device__ __forceinline__ void path_error(const TraceParams& tp, int slot) {
-    float* e = tp.path_err + 12 * (size_t)slot;
-#pragma unroll
-    for (int j = 0; j < 6; j++) e[j] = sqrtf(e[j] * e[j] + e[6 + j] * e[6 + j]);
-}
+// The field of the current state: 2 its component is known (E), 1 the state
+// is located (lane S holds its tetrahedron, b the coordinates), 0 neither.
+// Every trial of a step evaluates its first stage at the same point, so a
+// retried trial takes the field from here, and the first trial takes the
+// location from the one that accepted the state.
+struct Stage0 {
+    double E;
+    int tet;
+    int mode;
+};
 
 // One Cash-Karp trial step (o5_integrator, trajectory_3d.cpp:583-676) of
 // length dt from (x, v), its arithmetic in R: FP64, or FP32 as the reference
@@ -499,90 +521,95 @@ __device__ __forceinline__ void path_error(const TraceParams& tp, int slot) {
 // located and their fields interpolated as in FP64, then rounded to R.
 // *rel: the largest relative error of a position or velocity component (as
 // errorRestricted_stepper forms it, trajectory_3d.cpp:366-387).  Returns
-// false when a walk exceeded its bound.  s0: the first stage's field, kept
-// across the trials of a step.
-// The stages run as a loop that is not unrolled, the tableau's rows read from
-// constant memory: the kernel then holds one copy of the point location and
-// interpolation in its hot loop instead of six.  A flight is a long chain of
-// dependent steps on few warps per SM, and the unrolled body stalled on
-// instruction fetch more than on anything else; the arithmetic, and so every
-// result, is the same.
-__constant__ double kCashKarpB[6][5] = {{0, 0, 0, 0, 0},
-                                        {1.0 / 5.0, 0, 0, 0, 0},
-                                        {3.0 / 40.0, 9.0 / 40.0, 0, 0, 0},
-                                        {3.0 / 10.0, -9.0 / 10.0, 6.0 / 5.0, 0, 0},
-                                        {-11.0 / 54.0, 5.0 / 2.0, -70.0 / 27.0, 35.0 / 27.0, 0},
-                                        {1631.0 / 55296.0, 175.0 / 512.0, 575.0 / 13824.0, 44275.0 / 110592.0,
-                                         253.0 / 4096.0}};
-// The first stage's field of the current state.  Every trial of a step
-// evaluates its first stage at the same point, so a retried trial (after the
-// stepper shrank dt) takes the field from here and starts its next walk from
-// the tetrahedron it was found in.  The tetrahedron holding a point does not
-// depend on where a walk to it starts (short of a point on a shared face,
-// where both sides interpolate the same field), so the flights are those of
-// the recomputation; on 4096 probe ions in each precision they were
-// identical bit for bit.
-struct Stage0 {
-    V3 E;
-    int tet;
-    bool have;
-};
+// false when a walk exceeded its bound.
+// A lane holds one component (c) of every vector.  The position of stage b
+// takes the increments h v_j of the stages before it, and v_j the fields of
+// the stages before j: so position b does not wait for the field of stage
+// b - 1, and the stages go in three rounds of two whose points are located
+// and interpolated together.  Each later stage's sums take the increments as
+// they come, in stage order, as one sum over them would.
 template <typename R>
-__device__ __forceinline__ bool ck_trial(const DevMesh& m, TetCache& fc, const TraceParams& tp, unsigned& rot, int& cur,
-                                         V3 x, V3 v, double k, double dt, V3* nxo, V3* nvo, V3* exo, V3* evo,
+__device__ __forceinline__ bool ck_trial(const DevMesh& m, LaneTet& T, int lane, int c, int& S, int& next, Bary& b,
+                                         const TraceParams& tp, unsigned& rot, bool direct, double xc, double vc,
+                                         double k, double dt, double* nxo, double* nvo, double* exo, double* evo,
                                          double* relo, Stage0& s0) {
-    constexpr double C5[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0, 0.0, 512.0 / 1771.0};
-    constexpr double C4[6] = {2825.0 / 27648.0, 0.0, 18575.0 / 48384.0, 13525.0 / 55296.0, 277.0 / 14336.0, 1.0 / 4.0};
-    const R xx = (R)x.x, xy = (R)x.y, xz = (R)x.z, vx = (R)v.x, vy = (R)v.y, vz = (R)v.z;
-    const R kk = (R)k, h = (R)dt;
-    R dx[6][3], dv[6][3];
+    const R xx = (R)xc, vv = (R)vc, kk = (R)k, h = (R)dt;
+    R sx[6] = {xx, xx, xx, xx, xx, xx}, sv[6] = {vv, vv, vv, vv, vv, vv};
+    R nx = xx, nv = vv, ex = 0, ev = 0;
     bool walkOk = true;
 #pragma unroll 1
-    for (int s = 0; s < 6; s++) {
-        R px = xx, py = xy, pz = xz, qx = vx, qy = vy, qz = vz;
-#pragma unroll 1
-        for (int j = 0; j < s; j++) {
-            const R b = (R)kCashKarpB[s][j];
-            px += b * dx[j][0]; py += b * dx[j][1]; pz += b * dx[j][2];
-            qx += b * dv[j][0]; qy += b * dv[j][1]; qz += b * dv[j][2];
+    for (int r = 0; r < 3; r++) {
+        const R dxa = sv[0] * h;
+        const R wab = ck_coef<R>(r, 0);
+        const V3 pa = gather3((double)sx[0]);
+        const V3 pb = gather3((double)(sx[1] + wab * dxa));
+        const int known = r == 0 ? s0.mode : 0;
+        int Sa = S, ra = 0, rb = 0;
+        bool ina = false, inb = false;
+        if (known == 2) {
+            // the walk to b starts from the state's tetrahedron if the warp
+            // still holds it
+            const unsigned have = __ballot_sync(0xffffffffu, T.t == s0.tet);
+            if (have) S = __ffs((int)have) - 1;
         }
-        V3 E;
-        if (s == 0 && s0.have) {
-            E = s0.E;
-            cur = s0.tet;
-        } else {
-            walkOk &= fast_field(m, fc, V3{(double)px, (double)py, (double)pz}, cur, tp.walk_limit, rot, &E, &cur);
-            if (s == 0) {
-                s0.E = E;
-                s0.tet = cur;
-                s0.have = true;
+        Bary bb = lane_bary(T, pb, &inb);
+        if (known == 0) {
+            b = lane_bary(T, pa, &ina);
+            const unsigned hit = direct ? 0u : __ballot_sync(0xffffffffu, ina);
+            if (hit) {
+                S = __ffs((int)hit) - 1;
+            } else {
+                const int from = S;
+                ra = warp_walk(m, T, lane, S, next, -1, pa, b, pb, bb, inb, tp.walk_limit, rot);
+                if (ra < 0) S = from;
+            }
+            Sa = S;
+        }
+        {
+            const unsigned hit = direct ? 0u : __ballot_sync(0xffffffffu, inb);
+            if (hit) {
+                S = __ffs((int)hit) - 1;
+            } else {
+                const int from = S;
+                rb = warp_walk(m, T, lane, S, next, Sa, pb, bb, pa, b, ina, tp.walk_limit, rot);
+                if (rb < 0) S = from;
             }
         }
-        dv[s][0] = (R)E.x * kk * h; dv[s][1] = (R)E.y * kk * h; dv[s][2] = (R)E.z * kk * h;
-        dx[s][0] = qx * h; dx[s][1] = qy * h; dx[s][2] = qz * h;
-    }
-    R nx[3] = {xx, xy, xz}, nv[3] = {vx, vy, vz}, ex[3] = {0, 0, 0}, ev[3] = {0, 0, 0};
+        walkOk = walkOk && ra != -2 && rb != -2;
+        if ((lane == Sa && ra == 0 && known != 2) || (lane == S && rb == 0)) lane_load_fields(m, T);
+        double Ea = lane_field(T, b, Sa, c);
+        if (known == 2) Ea = s0.E;
+        else if (ra < 0) Ea = 0.0;
+        double Eb = lane_field(T, bb, S, c);
+        if (rb < 0) Eb = 0.0;
+        if (r == 0) {
+            s0.tet = __shfl_sync(0xffffffffu, T.t, Sa);
+            s0.E = Ea;
+            s0.mode = 2;
+        }
+        const R dva = (R)Ea * kk * h, dvb = (R)Eb * kk * h;
+        const R dxb = (sv[1] + wab * dva) * h;
+        const R c5a = ck_coef<R>(r, 9), c5b = ck_coef<R>(r, 10), dca = ck_coef<R>(r, 11), dcb = ck_coef<R>(r, 12);
+        nx += c5a * dxa; nv += c5a * dva; ex += dca * dxa; ev += dca * dva;
+        nx += c5b * dxb; nv += c5b * dvb; ex += dcb * dxb; ev += dcb * dvb;
 #pragma unroll
-    for (int s = 0; s < 6; s++) {
-        const R c5 = (R)C5[s], dc = (R)(C5[s] - C4[s]);
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            nx[c] += c5 * dx[s][c];
-            nv[c] += c5 * dv[s][c];
-            ex[c] += dc * dx[s][c];
-            ev[c] += dc * dv[s][c];
+        for (int j = 0; j < 4; j++) {
+            const R wa = ck_coef<R>(r, 1 + j), wb = ck_coef<R>(r, 5 + j);
+            sx[j] = sx[j + 2] + wa * dxa;
+            sv[j] = sv[j + 2] + wa * dva;
+            sx[j] += wb * dxb;
+            sv[j] += wb * dvb;
         }
     }
     R rel = 0;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        if (nx[c] != (R)0) rel = fmax(rel, fabs(ex[c] / nx[c]));
-        if (nv[c] != (R)0) rel = fmax(rel, fabs(ev[c] / nv[c]));
-    }
-    *nxo = V3{(double)nx[0], (double)nx[1], (double)nx[2]};
-    *nvo = V3{(double)nv[0], (double)nv[1], (double)nv[2]};
-    *exo = V3{(double)ex[0], (double)ex[1], (double)ex[2]};
-    *evo = V3{(double)ev[0], (double)ev[1], (double)ev[2]};
+    if (nx != (R)0) rel = fmax(rel, fabs(ex / nx));
+    if (nv != (R)0) rel = fmax(rel, fabs(ev / nv));
+    rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, 1));
+    rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, 2));
+    *nxo = (double)nx;
+    *nvo = (double)nv;
+    *exo = (double)ex;
+    *evo = (double)ev;
     *relo = (double)rel;
     return walkOk;
 }
@@ -605,20 +632,35 @@ __device__ __forceinline__ bool error_rule(double relIn, const TraceParams& tp, 
     return accept;
 }
 
-// One ion from x0 (velocity v0, charge/mass k) into *out; with kPath its
-// path and error estimate go to slot `slot` of tp's path buffers (a
-// separate instantiation, so that the flights without a path keep their
+// One ion from x (velocity v, charge/mass k) into *out, by one warp; with
+// kPath its path and error estimate go to slot `slot` of tp's path buffers
+// (a separate instantiation, so that the flights without a path keep their
 // registers).
 // kPrec: the arithmetic of the Cash-Karp steps (TraceParams::precision),
 // fixed per instantiation so that each kernel holds only its own registers.
+//
+// A flight is a chain of trial steps, each a chain of point locations and
+// interpolations, so what counts is the length of that chain.  Every lane
+// keeps the record (and vertex fields) of one of the last 32 tetrahedra the
+// flight came through, and a point is located by all lanes testing theirs at
+// once: 60% of the trials are retries with a smaller step, whose points lie
+// in tetrahedra already there, and so do most points of a step that is not
+// the first through a region.  Only a point in none of them walks on
+// (warp_walk), over the lanes' records where the walk crosses them.
+// Measured on the B200: 500 mixed-precision ions on a 307k-cell tip 12.9 ms
+// with one thread per ion, 5.7 ms so; 4096 FP64 ions on a 500k-cell alloy tip
+// 41.2 and 14.6 ms; the impacts the same to the bit.  About 1400 warp
+// instructions per trial at 5 cycles each (2.2 of them waits on the fixed
+// latency of dependent FP64 arithmetic), instead of 3400.  At 240 registers
+// eight warps fit an SM; 12 or 16 spilled and were slower (8.6 and 10.4
+// against 7.4 ms for 1000 ions).
 template <bool kPath, int kPrec>
 __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k, int guessTet, const TraceParams& tp,
                                           unsigned rot, int slot, ImpactOut* out) {
+    const int lane = threadIdx.x & 31;
+    const int c = min(lane & 3, 2);  // the lane's component of the state
     const V3 x0 = x;
     ImpactOut res;
-    TetCache fc;
-    fc.a.t = -1;
-    fc.a.hasF = false;
     double time = 0.0;
     int tet = locate(m, x, guessTet, tp.walk_limit, rot);
     res.steps = 0;
@@ -628,40 +670,59 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
     res.last_phi = 0.0f;
     if (kPath) {
         float* e = tp.path_err + 12 * (size_t)slot;
-#pragma unroll
-        for (int j = 0; j < 12; j++) e[j] = 0.0f;
-        if (tet >= 0) path_point(tp, slot, 0, 0.0, x, v, tet);  // Trajectory_3d::init (:99-123)
+        if (lane < 12) e[lane] = 0.0f;
+        if (lane == 0 && tet >= 0) path_point(tp, slot, 0, 0.0, x, v, tet);  // Trajectory_3d::init (:99-123)
+        __syncwarp();
     }
     if (tet < 0) {
         if (tet == -2) atomicOr(m.status, S_WALK_LIMIT);
         res.status = -1;  // Trajectory_3d::init: initial point is outside
         res.stop[0] = (float)x.x; res.stop[1] = (float)x.y; res.stop[2] = (float)x.z;
         res.stop_time = 0.0f;
-        *out = res;
+        if (lane == 0) *out = res;
         return;
     }
-    V3 E0;
-    int cur = tet;  // tetrahedron of the last located point: the next walk starts there
-    if (!fast_field(m, fc, x, tet, tp.walk_limit, rot, &E0, &cur)) atomicOr(m.status, S_WALK_LIMIT);
+    // a short bound on the walks keeps them as they are: each from the last
+    // located point's tetrahedron
+    const bool direct = tp.walk_limit < 64;
+    LaneTet T{};
+    T.t = -1;
+    int S = 0;     // the lane holding the last located point's tetrahedron
+    int next = 0;  // the slot filled last
+    Bary b{};      // every lane's coordinates of the current state, once it is located
+    if (lane == 0) {
+        load_slot(m, T, tet);
+        bool in;
+        b = lane_bary(T, x, &in);
+        if (T.vol6 == 0.0f) b.l0 = b.l1 = b.l2 = b.l3 = 0.25;
+        lane_load_fields(m, T);
+    }
+    double xc = c == 0 ? x.x : (c == 1 ? x.y : x.z), vc = c == 0 ? v.x : (c == 1 ? v.y : v.z);
+    Stage0 s0;
+    s0.E = lane_field(T, b, S, c);
+    s0.tet = tet;
+    s0.mode = 2;
     int status;
-    if (E0.x == 0.0 && E0.y == 0.0 && E0.z == 0.0) {
+    if (!__any_sync(0xffffffffu, s0.E != 0.0)) {
         status = 1;  // NO_FIELD
     } else {
         status = 3;  // ITERATION_LIMIT_PASSED unless another exit is taken
         double dt = tp.dt0;
+        bool loBefore = kPrec == 1;
         for (int it = 0; it < tp.max_steps; it++) {
-            V3 nx, nv;
+            double nxc = 0.0, nvc = 0.0;
             double used = dt;
             bool accepted = false;
-            bool located = false;  // the accepted trial point is already located (steppers 2, 3)
             int nt = -1;
+            V3 nx{};
             // FP32 arithmetic for this step: always with precision 1, and
             // with precision 2 once the ion is beyond fp64_radius of its start
             const double ddx = x.x - x0.x, ddy = x.y - x0.y, ddz = x.z - x0.z;
             const bool lo = kPrec != 0 && tp.integrator == 1 &&
                             (kPrec == 1 || ddx * ddx + ddy * ddy + ddz * ddz > tp.fp64_radius2);
-            Stage0 s0;
-            s0.have = false;
+            // the first step in FP32 starts from the state rounded to float
+            if (kPrec == 2 && lo != loBefore) s0.mode = 0;
+            loBefore = lo;
             for (int tries = 0; tries < tp.stepper_limit; tries++) {
                 res.trials++;
                 if (lo) {
@@ -670,42 +731,63 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
                     dt = tp.dt_min;
                 }
                 used = dt;
+                double rel = 0.0, exc = 0.0, evc = 0.0;
+                bool take = false;
                 if (tp.integrator == 0) {
                     // o1_integrator (trajectory_3d.cpp:560-581): Euler; the
                     // error estimate is the next state times dt^2
-                    V3 E;
-                    if (!fast_field(m, fc, x, cur, tp.walk_limit, rot, &E, &cur)) atomicOr(m.status, S_WALK_LIMIT);
-                    nv = V3{v.x + dt * E.x * k, v.y + dt * E.y * k, v.z + dt * E.z * k};
-                    nx = V3{x.x + dt * v.x, x.y + dt * v.y, x.z + dt * v.z};
-                    const bool any = nx.x != 0.0 || nx.y != 0.0 || nx.z != 0.0 || nv.x != 0.0 || nv.y != 0.0 ||
-                                     nv.z != 0.0;
-                    const double rel = any ? dt * dt : 0.0;
-                    const int verdict = stepper_verdict(m, fc, tp, nx, tet, cur, rot, rel, &dt, &nt, &located);
-                    if (verdict > 0) {
-                        accepted = true;
-                        break;
+                    if (s0.mode == 1) {
+                        if (lane == S) lane_load_fields(m, T);
+                        s0.E = lane_field(T, b, S, c);
+                        s0.mode = 2;
                     }
-                    continue;
+                    nvc = vc + dt * s0.E * k;
+                    nxc = xc + dt * vc;
+                    rel = __any_sync(0xffffffffu, nxc != 0.0 || nvc != 0.0) ? dt * dt : 0.0;
+                    exc = nxc * (used * used);
+                    evc = nvc * (used * used);
+                } else {
+                    bool walkOk;
+                    if (kPrec == 1 || (kPrec == 2 && lo))
+                        walkOk = ck_trial<float>(m, T, lane, c, S, next, b, tp, rot, direct, xc, vc, k, dt, &nxc, &nvc,
+                                                 &exc, &evc, &rel, s0);
+                    else
+                        walkOk = ck_trial<double>(m, T, lane, c, S, next, b, tp, rot, direct, xc, vc, k, dt, &nxc,
+                                                  &nvc, &exc, &evc, &rel, s0);
+                    if (!walkOk && lane == 0) atomicOr(m.status, S_WALK_LIMIT);
                 }
-                V3 ex, evv;
-                double rel;
-                bool walkOk;
-                if (kPrec == 1) walkOk = ck_trial<float>(m, fc, tp, rot, cur, x, v, k, dt, &nx, &nv, &ex, &evv, &rel, s0);
-                else if (kPrec == 0) walkOk = ck_trial<double>(m, fc, tp, rot, cur, x, v, k, dt, &nx, &nv, &ex, &evv, &rel, s0);
-                else walkOk = lo ? ck_trial<float>(m, fc, tp, rot, cur, x, v, k, dt, &nx, &nv, &ex, &evv, &rel, s0)
-                                 : ck_trial<double>(m, fc, tp, rot, cur, x, v, k, dt, &nx, &nv, &ex, &evv, &rel, s0);
-                if (!walkOk) atomicOr(m.status, S_WALK_LIMIT);
-                if (kPath) path_trial_error(tp, slot, ex, evv);
-                if (tp.stepper != 1) {
-                    const int verdict = stepper_verdict(m, fc, tp, nx, tet, cur, rot, rel, &dt, &nt, &located);
-                    if (verdict > 0) {
-                        accepted = true;
-                        break;
-                    }
-                    continue;
+                if (kPath && lane < 3) {
+                    // the latest trial's error vector
+                    float* e = tp.path_err + 12 * (size_t)slot + 6;
+                    e[c] = (float)exc;
+                    e[3 + c] = (float)evc;
                 }
-                if (kPrec == 0 ? error_rule<double>(rel, tp, &dt)
-                               : (lo ? error_rule<float>(rel, tp, &dt) : error_rule<double>(rel, tp, &dt))) {
+                const bool errorRule = tp.stepper == 1 && tp.integrator != 0;
+                const bool byTet = tp.stepper == 2 || tp.stepper == 3;  // verdicts that look at the tetrahedron
+                if (!byTet) {
+                    if (!errorRule) take = stepper_verdict(m, tp, tet, -1, rel, &dt);
+                    else if (kPrec == 0) take = error_rule<double>(rel, tp, &dt);
+                    else take = lo ? error_rule<float>(rel, tp, &dt) : error_rule<double>(rel, tp, &dt);
+                    if (!take) continue;
+                }
+                // the trial point located, for the verdict or the next step
+                nx = gather3(nxc);
+                bool in;
+                b = lane_bary(T, nx, &in);
+                const unsigned hit = direct ? 0u : __ballot_sync(0xffffffffu, in);
+                if (hit) {
+                    S = __ffs((int)hit) - 1;
+                    nt = 0;
+                } else {
+                    const int from = S;
+                    Bary bo;
+                    nt = warp_walk(m, T, lane, S, next, -1, nx, b, nx, bo, in, tp.walk_limit, rot);
+                    if (nt < 0) S = from;
+                }
+                if (nt == -2 && lane == 0) atomicOr(m.status, S_WALK_LIMIT);
+                if (nt == 0) nt = __shfl_sync(0xffffffffu, T.t, S);
+                if (byTet) take = stepper_verdict(m, tp, tet, nt, rel, &dt);
+                if (take) {
                     accepted = true;
                     break;
                 }
@@ -714,41 +796,42 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
                 status = 2;  // STEPPER_LIMIT_PASSED
                 break;
             }
-            if (!located) {
-                const int nsl = locate_cached(m, fc, nx, cur, tp.walk_limit, rot);
-                nt = nsl >= 0 ? fc.a.t : nsl;
-                if (nt == -2) atomicOr(m.status, S_WALK_LIMIT);
-            }
             res.steps++;
             if (kPath) {
-                // the error of the accepted step: o1_integrator's is the new
-                // state times dt^2 (trajectory_3d.cpp:568-576)
-                if (tp.integrator == 0) {
-                    const double d2 = used * used;
-                    path_trial_error(tp, slot, V3{nx.x * d2, nx.y * d2, nx.z * d2}, V3{nv.x * d2, nv.y * d2, nv.z * d2});
+                // Trajectory_3d::cumulative_error (trajectory_3d.cpp:683-700)
+                // with the accepted step's error: each of the six components
+                // becomes sqrt(current^2 + step^2), in float as the reference
+                // keeps it
+                __syncwarp();
+                if (lane < 6) {
+                    float* e = tp.path_err + 12 * (size_t)slot;
+                    e[lane] = sqrtf(e[lane] * e[lane] + e[6 + lane] * e[6 + lane]);
                 }
-                path_error(tp, slot);
-                path_point(tp, slot, res.steps, time + used, nx, nv, nt);
+                const V3 nv = gather3(nvc);
+                if (lane == 0) path_point(tp, slot, res.steps, time + used, nx, nv, nt);
+                __syncwarp();
             }
             const double tnext = lo ? (double)((float)time + (float)used) : time + used;
             if (nt < 0) {
                 // left the mesh: the previous point is the last inside it
                 res.last_tet = tet;
                 res.last_pos[0] = (float)x.x; res.last_pos[1] = (float)x.y; res.last_pos[2] = (float)x.z;
-                x = nx;
-                v = nv;
-                time = tnext;
+            }
+            x = nx;
+            xc = nxc;
+            vc = nvc;
+            time = tnext;
+            tet = nt;
+            if (nt < 0) {
                 tet = -1;
                 status = 5;  // SYSTEM_LIMIT_PASSED
                 break;
             }
-            x = nx;
-            v = nv;
-            time = tnext;
-            tet = nt;
-            cur = nt;
+            s0.tet = nt;
+            s0.mode = 1;
         }
     }
+    v = gather3(vc);
     if (tet >= 0) {
         res.last_tet = tet;
         res.last_pos[0] = (float)x.x; res.last_pos[1] = (float)x.y; res.last_pos[2] = (float)x.z;
@@ -772,40 +855,35 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
         int pt = -1;
         if (tet >= 0 && isfinite(p.x) && isfinite(p.y) && isfinite(p.z)) {
             pt = locate(m, p, tet, tp.walk_limit, rot);
-            if (pt == -2) atomicOr(m.status, S_WALK_LIMIT);
+            if (pt == -2 && lane == 0) atomicOr(m.status, S_WALK_LIMIT);
         }
-        path_point(tp, slot, res.steps + 1, time + dtz, p, v, pt);
+        if (lane == 0) path_point(tp, slot, res.steps + 1, time + dtz, p, v, pt);
         const float fdt = (float)dtz;
-        if (fdt > 0.0f) {
+        if (fdt > 0.0f && lane == 0) {
             float* e = tp.path_err + 12 * (size_t)slot;
 #pragma unroll
             for (int j = 0; j < 3; j++) e[j] += fdt * e[3 + j];
         }
     }
-    *out = res;
+    if (lane == 0) *out = res;
 }
 
-// perWarp: the ions each warp carries (its first perWarp lanes; the rest
-// return at once).  A flight is a chain of dependent loads whose branches
-// (walk lengths, rejected steps) differ from ion to ion, so a warp runs its
-// lanes' flights largely one after another: few ions per warp over every
-// warp the SMs can hold beats full warps on a fraction of them.
+// One ion per warp, one warp per block: as the flights' lengths differ by an
+// order of magnitude, the blocks waiting take the place of each that ends.
 template <bool kPath, int kPrec>
-__global__ void k_trace(DevMesh m, int nIons, int perWarp, const float* start, const float* vel, const float* qm,
-                        const int32_t* guess, TraceParams tp, ImpactOut* out) {
-    const int lane = threadIdx.x & 31;
-    const int ion = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * perWarp + lane;
-    if (lane >= perWarp || ion >= nIons) return;
-    const V3 x{start[3 * ion], start[3 * ion + 1], start[3 * ion + 2]};
-    const V3 v = vel ? V3{vel[3 * ion], vel[3 * ion + 1], vel[3 * ion + 2]} : V3{0, 0, 0};
+__global__ void __launch_bounds__(32) k_trace(DevMesh m, int nIons, const float* start, const float* vel,
+                                              const float* qm, const int32_t* guess, TraceParams tp, ImpactOut* out) {
+    const int ion = blockIdx.x;
+    if (ion >= nIons) return;
+    const V3 x{start[3 * (size_t)ion], start[3 * (size_t)ion + 1], start[3 * (size_t)ion + 2]};
+    const V3 v = vel ? V3{vel[3 * (size_t)ion], vel[3 * (size_t)ion + 1], vel[3 * (size_t)ion + 2]} : V3{0, 0, 0};
     trace_ion<kPath, kPrec>(m, x, v, qm[ion], guess ? guess[ion] : 0, tp, (unsigned)ion * 7u, ion, out + ion);
 }
 
-// A single ion from rest, its start passed by value (no staging copy)
+// A single ion, its start passed by value (no staging copy)
 template <bool kPath, int kPrec>
-__global__ void k_trace_one(DevMesh m, float x, float y, float z, float vx, float vy, float vz, float qm, int guess,
-                            TraceParams tp, ImpactOut* out) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__global__ void __launch_bounds__(32) k_trace_one(DevMesh m, float x, float y, float z, float vx, float vy, float vz,
+                                                  float qm, int guess, TraceParams tp, ImpactOut* out) {
     trace_ion<kPath, kPrec>(m, V3{x, y, z}, V3{vx, vy, vz}, qm, guess, tp, 0u, 0, out);
 }
 
@@ -825,18 +903,7 @@ void launch_trace(const DevMesh& m, int nIons, const float* start, const float* 
                   const int32_t* guess, TraceParams tp, ImpactOut* out, cudaStream_t s) {
     if (nIons <= 0) return;
     count_launch();
-    // ions per warp: as few as fill every warp slot the SMs hold at this
-    // kernel's register count (one wave), one warp per block
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto go = [&](auto kernel) {
-        int perSM = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, 32, 0) != cudaSuccess || perSM < 1) perSM = 1;
-        const long long slots = (long long)perSM * sms;
-        const int perWarp = (int)std::min<long long>(32, std::max<long long>(1, (nIons + slots - 1) / slots));
-        const int warps = (nIons + perWarp - 1) / perWarp;
-        kernel<<<warps, 32, 0, s>>>(m, nIons, perWarp, start, vel, qm, guess, tp, out);
-    };
+    auto go = [&](auto kernel) { kernel<<<nIons, 32, 0, s>>>(m, nIons, start, vel, qm, guess, tp, out); };
     const int prec = tp.precision == 1 ? 1 : (tp.precision == 2 ? 2 : 0);
     if (tp.path) {
         if (prec == 0) go(k_trace<true, 0>); else if (prec == 1) go(k_trace<true, 1>); else go(k_trace<true, 2>);
