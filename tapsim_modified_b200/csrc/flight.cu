@@ -171,8 +171,8 @@ __global__ void k_vertex_fields(DevMesh m, const int32_t* __restrict__ cells, in
 // six-fold volume (float), the gradients n1, n2, n3 of the barycentric
 // coordinates of vertices 1..3 (9 doubles: lambda_k(p) = n_k.(p - v0),
 // lambda_0 = 1 - lambda_1 - lambda_2 - lambda_3), the neighbours (4 ints)
-// and the vertex ids (4 ints).  A walk step then tests the four faces with
-// three dot products, and the same lambdas are the interpolation weights
+// the vertex ids (4 ints) and 3e-13 times the largest gradient component
+// (double).  A walk step then tests the four faces with three dot products, and the same lambdas are the interpolation weights
 // |sub-volume| / volume of tetWeights (geometry_3d.cpp:916-980).  A flat
 // tetrahedron stores zero gradients and volume 0.
 constexpr int kTetWords = 32;
@@ -208,7 +208,9 @@ __global__ void k_pack_tets(DevMesh m, float* pack) {
         oi[22 + k] = m.tet_n[4 * t + k];
         oi[26 + k] = v[k];
     }
-    oi[30] = oi[31] = 0;
+    double gmax = 0.0;
+    for (int k = 0; k < 9; k++) gmax = fmax(gmax, fabs(g[k]));
+    reinterpret_cast<double*>(o)[15] = 3e-13 * gmax;
 }
 
 __device__ V3 vertex_field(const DevMesh& m, int i) {
@@ -249,17 +251,14 @@ __device__ __forceinline__ void load_slot(const DevMesh& m, LaneTet& s, int t) {
     const double2 g3 = __ldg(reinterpret_cast<const double2*>(p + 4));
     const double2 g4 = __ldg(reinterpret_cast<const double2*>(p + 5));  // g[8], neighbours 0, 1
     const int4 q6 = __ldg(reinterpret_cast<const int4*>(p + 6));       // neighbours 2, 3, vertices 0, 1
-    const int4 q7 = __ldg(reinterpret_cast<const int4*>(p + 7));       // vertices 2, 3, padding
+    const int4 q7 = __ldg(reinterpret_cast<const int4*>(p + 7));       // vertices 2, 3, gmax
     s.t = t;
     s.P0 = V3{q0.x, q0.y, q0.z};
     s.vol6 = q0.w;
     s.G1 = V3{g0.x, g0.y, g1.x};
     s.G2 = V3{g1.y, g2.x, g2.y};
     s.G3 = V3{g3.x, g3.y, g4.x};
-    const double m1 = fmax(fmax(fabs(s.G1.x), fabs(s.G1.y)), fabs(s.G1.z));
-    const double m2 = fmax(fmax(fabs(s.G2.x), fabs(s.G2.y)), fabs(s.G2.z));
-    const double m3 = fmax(fmax(fabs(s.G3.x), fabs(s.G3.y)), fabs(s.G3.z));
-    s.gmax = 3e-13 * fmax(m1, fmax(m2, m3));
+    s.gmax = __hiloint2double(q7.w, q7.z);
     const long long nb01 = __double_as_longlong(g4.y);
     s.nb0 = (int)(unsigned)(nb01 & 0xffffffffll);
     s.nb1 = (int)(unsigned)((unsigned long long)nb01 >> 32);
@@ -306,28 +305,55 @@ __device__ __noinline__ int face_side_exact(const float* xyz, double snap, int i
 }
 
 // The neighbour through which a walk to p leaves this lane's tetrahedron
-// (-1: the hull), kHere when p lies beyond none of its faces.  The faces are
-// tried in an order rotating from walk step to walk step.  A barycentric
-// coordinate decides its face unless it is within its rounding bound of
+// (-1: the hull), kHere when p lies beyond none of its faces.  Mostly every
+// coordinate is clear of lane_bary's bound, and the walk takes the face that
+// p is furthest beyond (in coordinates), the faces beyond which it lies in
+// an order rotating from step to step once the walk is long.  Otherwise a
+// coordinate decides its face unless it is within its own rounding bound of
 // zero (about a thousand ulps of the terms summed), or the tetrahedron is
 // flat; then the exact predicate decides.
+// For a point within a mesh quantum of a face, the coordinates may put it on
+// the other side than the predicate, which snaps the point to the mesh's
+// grid, and tetrahedra that decide differently can send a walk round in
+// circles.  A walk of kSnapStep steps goes on by the predicate on the snapped
+// point alone, whose decisions agree, so that it ends.
+constexpr int kSnapStep = 256;
 constexpr int kHere = -3;
-__device__ __forceinline__ int walk_exit(const DevMesh& m, const LaneTet& S, V3 p, const Bary& b, unsigned rot) {
+__device__ __forceinline__ int walk_exit(const DevMesh& m, const LaneTet& S, V3 p, const Bary& b, int step,
+                                         unsigned rot) {
     const double dx = p.x - S.P0.x, dy = p.y - S.P0.y, dz = p.z - S.P0.z;
-    const double a1 = fabs(S.G1.x * dx) + fabs(S.G1.y * dy) + fabs(S.G1.z * dz);
-    const double a2 = fabs(S.G2.x * dx) + fabs(S.G2.y * dy) + fabs(S.G2.z * dz);
-    const double a3 = fabs(S.G3.x * dx) + fabs(S.G3.y * dy) + fabs(S.G3.z * dz);
-    const double e1 = 1e-13 * a1, e2 = 1e-13 * a2, e3 = 1e-13 * a3, e0 = 1e-13 * (1.0 + a1 + a2 + a3);
-    unsigned out = (b.l0 < -e0 ? 1u : 0u) | (b.l1 < -e1 ? 2u : 0u) | (b.l2 < -e2 ? 4u : 0u) | (b.l3 < -e3 ? 8u : 0u);
-    unsigned sure = out | (b.l0 > e0 ? 1u : 0u) | (b.l1 > e1 ? 2u : 0u) | (b.l2 > e2 ? 4u : 0u) |
-                    (b.l3 > e3 ? 8u : 0u);
-    if (S.vol6 == 0.0f) out = sure = 0u;
-    for (unsigned left = ~sure & 15u; left; left &= left - 1u) {
-        const int k = __ffs((int)left) - 1;
-        const int i0 = pick4(kFaceDev[k][0], S.v0, S.v1, S.v2, S.v3);
-        const int i1 = pick4(kFaceDev[k][1], S.v0, S.v1, S.v2, S.v3);
-        const int i2 = pick4(kFaceDev[k][2], S.v0, S.v1, S.v2, S.v3);
-        if (face_side_exact(m.xyz, m.snap, i0, i1, i2, p) < 0) out |= 1u << k;
+    const double thr = S.gmax * (fabs(dx) + fabs(dy) + fabs(dz)) + 1e-13;
+    unsigned out = (b.l0 < -thr ? 1u : 0u) | (b.l1 < -thr ? 2u : 0u) | (b.l2 < -thr ? 4u : 0u) |
+                   (b.l3 < -thr ? 8u : 0u);
+    const bool clear = fabs(b.l0) > thr && fabs(b.l1) > thr && fabs(b.l2) > thr && fabs(b.l3) > thr;
+    const bool exact = S.vol6 == 0.0f || step >= kSnapStep;
+    if (clear && !exact && step < 24) {
+        if (out == 0u) return kHere;
+        double low = b.l0;
+        int to = S.nb0;
+        if (b.l1 < low) { low = b.l1; to = S.nb1; }
+        if (b.l2 < low) { low = b.l2; to = S.nb2; }
+        if (b.l3 < low) to = S.nb3;
+        return to;
+    }
+    if (!clear || exact) {
+        const double a1 = fabs(S.G1.x * dx) + fabs(S.G1.y * dy) + fabs(S.G1.z * dz);
+        const double a2 = fabs(S.G2.x * dx) + fabs(S.G2.y * dy) + fabs(S.G2.z * dz);
+        const double a3 = fabs(S.G3.x * dx) + fabs(S.G3.y * dy) + fabs(S.G3.z * dz);
+        const double e1 = 1e-13 * a1, e2 = 1e-13 * a2, e3 = 1e-13 * a3, e0 = 1e-13 * (1.0 + a1 + a2 + a3);
+        out = (b.l0 < -e0 ? 1u : 0u) | (b.l1 < -e1 ? 2u : 0u) | (b.l2 < -e2 ? 4u : 0u) | (b.l3 < -e3 ? 8u : 0u);
+        unsigned sure = out | (b.l0 > e0 ? 1u : 0u) | (b.l1 > e1 ? 2u : 0u) | (b.l2 > e2 ? 4u : 0u) |
+                        (b.l3 > e3 ? 8u : 0u);
+        V3 q = p;
+        if (exact) out = sure = 0u;
+        if (step >= kSnapStep) q = V3{rint(p.x * m.snap) / m.snap, rint(p.y * m.snap) / m.snap, rint(p.z * m.snap) / m.snap};
+        for (unsigned left = ~sure & 15u; left; left &= left - 1u) {
+            const int k = __ffs((int)left) - 1;
+            const int i0 = pick4(kFaceDev[k][0], S.v0, S.v1, S.v2, S.v3);
+            const int i1 = pick4(kFaceDev[k][1], S.v0, S.v1, S.v2, S.v3);
+            const int i2 = pick4(kFaceDev[k][2], S.v0, S.v1, S.v2, S.v3);
+            if (face_side_exact(m.xyz, m.snap, i0, i1, i2, q) < 0) out |= 1u << k;
+        }
     }
     if (out == 0u) return kHere;
     const unsigned r = rot & 3u;
@@ -346,7 +372,7 @@ __device__ __forceinline__ int warp_walk(const DevMesh& m, LaneTet& T, int lane,
                                          Bary& b, V3 other, Bary& bo, bool& inOther, int limit, unsigned& rot) {
     for (int step = 0; step < limit; step++) {
         int to = kHere;
-        if (lane == S) to = walk_exit(m, T, p, b, rot);
+        if (lane == S) to = walk_exit(m, T, p, b, step, rot);
         rot++;
         to = __shfl_sync(0xffffffffu, to, S);
         if (to == kHere) {
@@ -577,9 +603,11 @@ __device__ __forceinline__ bool ck_trial(const DevMesh& m, LaneTet& T, int lane,
         }
         walkOk = walkOk && ra != -2 && rb != -2;
         if ((lane == Sa && ra == 0 && known != 2) || (lane == S && rb == 0)) lane_load_fields(m, T);
-        double Ea = lane_field(T, b, Sa, c);
-        if (known == 2) Ea = s0.E;
-        else if (ra < 0) Ea = 0.0;
+        double Ea = s0.E;
+        if (known != 2) {
+            Ea = lane_field(T, b, Sa, c);
+            if (ra < 0) Ea = 0.0;
+        }
         double Eb = lane_field(T, bb, S, c);
         if (rb < 0) Eb = 0.0;
         if (r == 0) {
@@ -601,11 +629,14 @@ __device__ __forceinline__ bool ck_trial(const DevMesh& m, LaneTet& T, int lane,
             sv[j] += wb * dvb;
         }
     }
+    // lanes 0..3 of every eight take the position's quotient, the others the
+    // velocity's
+    const R num = (lane & 4) ? ev : ex, den = (lane & 4) ? nv : nx;
     R rel = 0;
-    if (nx != (R)0) rel = fmax(rel, fabs(ex / nx));
-    if (nv != (R)0) rel = fmax(rel, fabs(ev / nv));
+    if (den != (R)0) rel = fmax(rel, fabs(num / den));
     rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, 1));
     rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, 2));
+    rel = fmax(rel, __shfl_xor_sync(0xffffffffu, rel, 4));
     *nxo = (double)nx;
     *nvo = (double)nv;
     *exo = (double)ex;
@@ -623,7 +654,11 @@ __device__ __forceinline__ bool error_rule(double relIn, const TraceParams& tp, 
     const R rel = (R)relIn, tol = (R)tp.tol;
     R dt = (R)*dtIo;
     const bool accept = rel < tol || dt == (R)tp.dt_min;
-    if (!accept || rel != (R)0) {
+    // the fourth root of a quotient below 0.9^-4 = 1.5242 leaves tmp below
+    // dt, so that an accepted step's dt grows by 1.1 whatever the root
+    if (accept && rel != (R)0 && tol < rel * (R)1.52) {
+        dt = dt * (R)1.1;
+    } else if (!accept || rel != (R)0) {
         const R tmp = dt * (R)pow(tol / rel, (R)0.25) * (R)0.9;
         if (accept) dt = tmp < dt ? dt * (R)1.1 : tmp;
         else dt = tmp > dt ? dt * (R)0.9 : tmp;
@@ -647,9 +682,9 @@ __device__ __forceinline__ bool error_rule(double relIn, const TraceParams& tp, 
 // in tetrahedra already there, and so do most points of a step that is not
 // the first through a region.  Only a point in none of them walks on
 // (warp_walk), over the lanes' records where the walk crosses them.
-// Measured on the B200: 500 mixed-precision ions on a 307k-cell tip 12.9 ms
-// with one thread per ion, 5.7 ms so; 4096 FP64 ions on a 500k-cell alloy tip
-// 41.2 and 14.6 ms; the impacts the same to the bit.  About 1400 warp
+// Measured on the B200: 1000 mixed-precision ions on a 307k-cell tip 15.2 ms
+// with one thread per ion, 6.2 ms so; 4096 FP64 ions on a 500k-cell alloy tip
+// 40.3 and 13.2 ms; the impacts the same to the bit.  About 1300 warp
 // instructions per trial at 5 cycles each (2.2 of them waits on the fixed
 // latency of dependent FP64 arithmetic), instead of 3400.  At 240 registers
 // eight warps fit an SM; 12 or 16 spilled and were slower (8.6 and 10.4
@@ -684,7 +719,7 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
     }
     // a short bound on the walks keeps them as they are: each from the last
     // located point's tetrahedron
-    const bool direct = tp.walk_limit < 64;
+    const bool direct = tp.walk_limit < kSnapStep;
     LaneTet T{};
     T.t = -1;
     int S = 0;     // the lane holding the last located point's tetrahedron

@@ -1,7 +1,7 @@
 """Flights by one warp per ion: points found among the warp's tetrahedra
 against points found by walking alone.
 
-With a walk bound below 64 every point is located by a walk from the last
+With a walk bound below 256 every point is located by a walk from the last
 one's tetrahedron; above, by the tetrahedra the warp holds where one of them
 holds the point.  The tetrahedron found is the same unless the point lies on
 a shared face to rounding, so nearly every flight is the same to the bit, and
@@ -31,7 +31,7 @@ def test_located_and_walked_flights_agree(grid, ions, precision):
     pick = np.random.default_rng(5).choice(nodes, ions, replace=ions > len(nodes))
     kw = dict(precision=precision, fp64_radius=5e-9)
     hit = np.ctypeslib.as_array(g.trace(a["xyz"][pick], QM_FE, a["node_tet"][pick], **kw))
-    walked = np.ctypeslib.as_array(g.trace(a["xyz"][pick], QM_FE, a["node_tet"][pick], walk_limit=63, **kw))
+    walked = np.ctypeslib.as_array(g.trace(a["xyz"][pick], QM_FE, a["node_tet"][pick], walk_limit=255, **kw))
     assert np.all(hit["status"] == 5) and np.all(walked["status"] == 5)
     same = (hit["trials"] == walked["trials"]) & np.all(hit["stop"] == walked["stop"], axis=1)
     assert np.mean(same) >= 0.95
