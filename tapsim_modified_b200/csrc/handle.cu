@@ -222,6 +222,7 @@ struct tg_handle {
     cudaGraphExec_t cgExec[2] = {nullptr, nullptr};
     std::vector<uint64_t> cgKey[2];
     long long cgNodes[2] = {0, 0};
+    DBuf<int32_t> cgDone;                // [1] iterations of the last one-launch node-space solve
     DBuf<int32_t> cgIterDev;             // [1] their counter
     DBuf<double> cgTgtDev;               // [2] their targets rel2, abs2
     int lastItersJacobi = 16, lastItersAmg = 4;  // iterations of the last inner solves
@@ -908,6 +909,7 @@ void tg_destroy(tg_handle* h) {
     h->loopDone.release();
     for (int w = 0; w < 2; w++)
         if (h->cgExec[w]) cudaGraphExecDestroy(h->cgExec[w]);
+    h->cgDone.release();
     h->cgIterDev.release();
     h->cgTgtDev.release();
     if (h->captureStream) cudaStreamDestroy(h->captureStream);
@@ -1736,7 +1738,8 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
         rc = amg_setup(h, &inf.setup_seconds);
         if (rc != TG_OK) return rc;
     }
-    bool loopPending = false;  // a looped inner solve whose count is still on its way
+    // looped and one-launch inner solves whose counts are still on their way
+    bool loopPending = false, cgPending = false;
     for (int outer = 0;; outer++) {
         if (outer == 0 && incremental) {
             if (warm && !warmFirst) {
@@ -1766,6 +1769,12 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
             g_launches.fetch_add(h->loopNodes * k, std::memory_order_relaxed);
             h->lastItersAmg = k;
             loopPending = false;
+        }
+        if (cgPending) {
+            const int k = h->pin->loopIters[1];
+            inf.inner += k;
+            inf.inner_neumann += k;
+            cgPending = false;
         }
         // sums kept across removals can round to a little below zero
         r2[0] = std::max(r2[0], 0.0);
@@ -1797,13 +1806,25 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
             if (rc != TG_OK) return rc;
         }
         if (h->countAllN > 0) {
-            launch_vcg_couple_neumann(m, vsys, h->allN.p, h->countAllN, vN.r, h->stream, fp64);
             // the Neumann rows' share of the global residual only has to fall
             // below 0.3 of the outer tolerance (the V rows' solve brings
             // theirs to about the same), whatever their own start
             const double floorN = 0.3 * o->rel_tol;
-            rc = run_cg(h, 1, h->allN.p, h->countAllN, rtol, o->max_inner, &itN, floorN * floorN * h->bnorm2);
-            if (rc != TG_OK) return rc;
+            const double floor2 = floorN * floorN * h->bnorm2;
+            // one launch up to kCgSolveRows rows; beyond, a grid of them (a
+            // cluster's eight SMs would be the bound)
+            cgPending = h->launchMode >= 1 && h->countAllN <= kCgSolveRows;
+            if (cgPending) {
+                if (!h->cgDone.p) CK(h->cgDone.alloc(1));
+                CK(launch_cg_solve(m, h->allN.p, h->countAllN, vN, vsys, fp64, rtol * rtol, floor2, o->max_inner,
+                                   h->cgDone.p, h->stream));
+                CK(cudaMemcpyAsync(&h->pin->loopIters[1], h->cgDone.p, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                   h->stream));
+            } else {
+                launch_vcg_couple_neumann(m, vsys, h->allN.p, h->countAllN, vN.r, h->stream, fp64);
+                rc = run_cg(h, 1, h->allN.p, h->countAllN, rtol, o->max_inner, &itN, floor2);
+                if (rc != TG_OK) return rc;
+            }
         }
         if (itV < 0) {
             loopPending = true;
@@ -1813,7 +1834,7 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
         inf.inner_neumann += itN;
         if (fp64) launch_vcg64_apply(m, vsys, h->vActive, fromEvent, h->stream);
         else launch_vcg_apply(m, vsys, h->vActive, fromEvent, h->stream);
-        launch_apply_correction(m, h->allN.p, h->countAllN, vN, h->stream);
+        if (!cgPending) launch_apply_correction(m, h->allN.p, h->countAllN, vN, h->stream);
     }
     h->selValid = false;
     h->converged = true;

@@ -260,6 +260,12 @@ void launch_cg_replay_step(int32_t* iter, cudaStream_t s);
 // max(rel2 * r.r at the start (scal[2]), abs2)
 void launch_cg_iter(const DevMesh& m, const int32_t* rows, int count, CGVectors v, int it, double rel2, double abs2,
                     cudaStream_t s);
+// the whole solve of the Neumann rows in one launch: launch_vcg_couple_neumann,
+// init, iterations and launch_apply_correction, for a list of at most
+// kCgSolveRows rows; *iters: the iterations taken
+constexpr int kCgSolveRows = 16384;
+cudaError_t launch_cg_solve(const DevMesh& m, const int32_t* rows, int count, CGVectors v, const VSys& vs, bool fromX64,
+                            double rel2, double abs2, int maxIter, int32_t* iters, cudaStream_t s);
 // the SpMV kernel of one CG iteration on its own (timing hook)
 void launch_cg_spmv_only(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s);
 // rhs_N += sum over non-Neumann free neighbours c_ij x_j (coupling of the

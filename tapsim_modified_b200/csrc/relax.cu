@@ -10,6 +10,10 @@
 //   other rows:    the same sums skipping Neumann neighbours
 // The skip is folded into ceff (0 for a Neumann neighbour of a non-Neumann
 // row), so every free row is phi_i = (sum_j ceff_ij phi_j - q_i) / diag_i.
+#include <cooperative_groups.h>
+
+#include <atomic>
+
 #include "kernels.cuh"
 
 namespace tgd {
@@ -207,6 +211,209 @@ __global__ void k_cg_replay_begin(int32_t* iter, double* tgt, double rel2, doubl
 }
 __global__ void k_cg_replay_step(int32_t* iter) { *iter += 1; }
 
+// The whole node-space CG solve of the Neumann rows in one launch of one
+// cluster: the V rows' correction taken into the right-hand side (as
+// k_vcg_couple_neumann takes it), the iterations of k_cg_spmv, k_cg_update
+// and k_cg_pupdate with the same arithmetic per row, their sums through
+// distributed shared memory and three cluster barriers in place of the
+// kernel boundaries, and the correction applied (as k_apply_correction);
+// *iters gets the iterations taken (as cg_met ends them).  The rows are a
+// few thousand (6,103 of the 307k-cell tip, 11,845 of the 835k-cell one): a
+// grid of them is a few blocks, and an iteration from replayed graphs was
+// launches and host reads, 34 us each.  Here every block keeps the whole of p
+// in shared memory, each thread its rows' couplings (to rows of the list; p
+// is zero elsewhere, and there are six on average) and the rest of their
+// state in registers.  What bounds an iteration is the barriers and each
+// warp's share of the reductions, so 512 threads a block with up to four
+// rows each beat 1024 with up to two (11,845 rows: 24 us an iteration).
+// Measured: the Neumann part of a 307k-cell tip's event (15 iterations, three
+// solves) 510 -> 150 us, of an 835k-cell tip's 370 -> 115 us.
+constexpr int kCgThreads = 512;
+constexpr int kCgCluster = 8;
+constexpr int kCgWarps = kCgCluster * kCgThreads / 32;
+// couplings per row kept in shared memory; a longer row reads its last ones
+// from global memory
+constexpr int kCgWidth = 12;
+constexpr size_t cg_solve_smem(int rowsPerThread) {
+    return rowsPerThread * (sizeof(float) * kCgCluster * kCgThreads +
+                            (sizeof(float) + sizeof(uint16_t)) * kCgWidth * kCgThreads);
+}
+
+// Sums over the cluster of one or two values per thread: every warp's sums
+// go to every block, and each warp adds them all in the same order.
+// parts[turn] is written again only after another barrier.
+template <bool kTwo>
+__device__ __forceinline__ void cluster_sum(cooperative_groups::cluster_group& cl, double (*parts)[2][kCgWarps],
+                                            int& turn, double& a, double& b) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (int)cl.block_rank() * (kCgThreads / 32) + (threadIdx.x >> 5);
+    a = warp_sum(a);
+    if (kTwo) b = warp_sum(b);
+    if (lane < kCgCluster) {
+        *cl.map_shared_rank(&parts[turn][0][warp], lane) = a;
+        if (kTwo) *cl.map_shared_rank(&parts[turn][1][warp], lane) = b;
+    }
+    cl.sync();
+    a = b = 0.0;
+#pragma unroll
+    for (int k = 0; k < kCgWarps / 32; k++) {
+        a += parts[turn][0][k * 32 + lane];
+        if (kTwo) b += parts[turn][1][k * 32 + lane];
+    }
+    a = warp_sum(a);
+    if (kTwo) b = warp_sum(b);
+    turn ^= 1;
+}
+
+template <int kRows>
+__global__ void __launch_bounds__(kCgThreads) k_cg_solve(DevMesh m, const int32_t* __restrict__ rows, int count,
+                                                         CGVectors v, const int32_t* __restrict__ slotOf,
+                                                         const float* __restrict__ xV, const double* __restrict__ xV64,
+                                                         double rel2, double abs2, int maxIter, int32_t* iters) {
+    constexpr int W = kCgWidth;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    extern __shared__ float p[];  // the whole of p, by position in the list
+    float* const val = p + kRows * kCgCluster * kCgThreads;
+    uint16_t* const idx = reinterpret_cast<uint16_t*>(val + W * kRows * kCgThreads);
+    __shared__ double parts[2][2][kCgWarps];
+    const int tid = threadIdx.x;
+    // position + 1 in the list by node (0: not in it), in the words of the
+    // vector A p, which is zero outside a solve
+    int32_t* const pos = reinterpret_cast<int32_t*>(v.ap);
+    int row[kRows], groups[kRows], more[kRows], end[kRows];
+    float x[kRows], r[kRows], z[kRows], pi[kRows], d[kRows];
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int t = (k * kCgCluster + (int)cl.block_rank()) * kCgThreads + tid;
+        row[k] = t < count ? rows[t] : -1;
+        if (row[k] >= 0) __stcg(pos + row[k], t + 1);
+    }
+    cl.sync();  // every block has started, and pos is complete
+    int turn = 0;
+    double rz = 0.0, rr = 0.0;
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        x[k] = r[k] = z[k] = pi[k] = 0.0f;
+        d[k] = 1.0f;
+        groups[k] = more[k] = end[k] = 0;
+        if (row[k] < 0) continue;
+        int q = m.row_ptr[row[k]], len = 0;
+        end[k] = m.row_ptr[row[k] + 1];
+        more[k] = end[k];
+        float s = 0.0f;
+        for (; q < end[k]; q += 4) {
+            int c[4], j[4], sl[4];
+            float a[4];
+            double xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool in = q + u < end[k];
+                c[u] = in ? m.col[q + u] : -1;
+                a[u] = in ? m.ceff32[q + u] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                j[u] = c[u] >= 0 ? __ldcg(pos + c[u]) : 0;
+                sl[u] = c[u] >= 0 ? slotOf[c[u]] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) xv[u] = sl[u] < 0 ? 0.0 : (xV64 ? xV64[sl[u]] : (double)xV[sl[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (sl[u] >= 0) s = fmaf(a[u], (float)xv[u], s);
+                if (j[u] == 0) continue;
+                if (len < W) {
+                    val[(k * W + len) * kCgThreads + tid] = a[u];
+                    idx[(k * W + len) * kCgThreads + tid] = (uint16_t)(j[u] - 1);
+                } else if (len == W) {
+                    more[k] = q + u;  // the couplings from here on stay in global memory
+                }
+                len++;
+            }
+        }
+        len = min(len, W);
+        groups[k] = (len + 3) / 4;
+        for (; len < 4 * groups[k]; len++) {  // padding: zero times the first row's p
+            val[(k * W + len) * kCgThreads + tid] = 0.0f;
+            idx[(k * W + len) * kCgThreads + tid] = 0;
+        }
+        r[k] = v.r[row[k]] + s;
+        d[k] = m.diag32[row[k]];
+        z[k] = pi[k] = r[k] / d[k];
+        rz += (double)r[k] * (double)z[k];
+        rr += (double)r[k] * (double)r[k];
+        const int t = (k * kCgCluster + (int)cl.block_rank()) * kCgThreads + tid;
+#pragma unroll
+        for (int b = 0; b < kCgCluster; b++) cl.map_shared_rank(p, b)[t] = pi[k];
+    }
+    cluster_sum<true>(cl, parts, turn, rz, rr);
+    const double target = fmax(rel2 * rr, abs2);
+    int it = 0;
+    while (it < maxIter && rr > target) {  // a NaN ends the solve
+        double pap = 0.0, none = 0.0;
+        float ap[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            float s = 0.0f;
+            for (int g = 0; g < groups[k]; g++) {
+                float a[4], pj[4];
+                int at[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    a[u] = val[(k * W + 4 * g + u) * kCgThreads + tid];
+                    at[u] = idx[(k * W + 4 * g + u) * kCgThreads + tid];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) pj[u] = p[at[u]];
+#pragma unroll
+                for (int u = 0; u < 4; u++) s = fmaf(a[u], pj[u], s);
+            }
+            for (int q = more[k]; q < end[k]; q++) {
+                const int j = __ldcg(pos + m.col[q]);
+                if (j > 0) s = fmaf(m.ceff32[q], p[j - 1], s);
+            }
+            ap[k] = fmaf(d[k], pi[k], -s);
+            pap += (double)pi[k] * (double)ap[k];
+        }
+        cluster_sum<false>(cl, parts, turn, pap, none);
+        const float alpha = pap > 0.0 ? (float)(rz / pap) : 0.0f;
+        double rzn = 0.0, rrn = 0.0;
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            x[k] = fmaf(alpha, pi[k], x[k]);
+            r[k] = fmaf(-alpha, ap[k], r[k]);
+            z[k] = r[k] / d[k];
+            rzn += (double)r[k] * (double)z[k];
+            rrn += (double)r[k] * (double)r[k];
+        }
+        cluster_sum<true>(cl, parts, turn, rzn, rrn);
+        const float beta = (float)(rzn / rz);
+        rz = rzn;
+        rr = rrn;
+        it++;
+        if (!(rr > target)) break;
+        // no block still reads the old p: all have passed pap's barrier
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            if (row[k] < 0) continue;
+            pi[k] = fmaf(beta, pi[k], z[k]);
+            const int t = (k * kCgCluster + (int)cl.block_rank()) * kCgThreads + tid;
+#pragma unroll
+            for (int b = 0; b < kCgCluster; b++) cl.map_shared_rank(p, b)[t] = pi[k];
+        }
+        cl.sync();
+    }
+    cl.sync();  // no block reads pos, or writes into another, any more
+#pragma unroll
+    for (int k = 0; k < kRows; k++)
+        if (row[k] >= 0) {
+            m.phi64[row[k]] += (double)x[k];
+            v.r[row[k]] = 0.0f;
+            __stcg(pos + row[k], 0);
+        }
+    if (cl.block_rank() == 0 && tid == 0) *iters = it;
+}
+
 __global__ void k_add_coupled(DevMesh m, const int32_t* __restrict__ rows, int count, const float* xV, float* r) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
@@ -348,6 +555,37 @@ void launch_cg_iter(const DevMesh& m, const int32_t* rows, int count, CGVectors 
     { count_launch(); k_cg_spmv<<<blocks(count), kBlock, 0, s>>>(m, rows, count, v, it, rel2, abs2); }
     { count_launch(); k_cg_update<<<blocks(count), kBlock, 0, s>>>(m, rows, count, v, it, rel2, abs2); }
     { count_launch(); k_cg_pupdate<<<blocks(count), kBlock, 0, s>>>(rows, count, v, it, rel2, abs2); }
+}
+cudaError_t launch_cg_solve(const DevMesh& m, const int32_t* rows, int count, CGVectors v, const VSys& vs, bool fromX64,
+                            double rel2, double abs2, int maxIter, int32_t* iters, cudaStream_t s) {
+    static_assert(kCgSolveRows == 4 * kCgCluster * kCgThreads, "four rows per thread at most");
+    auto go = [&](auto kernel, int rowsPerThread, std::atomic<uint64_t>& done) -> cudaError_t {
+        const size_t smem = cg_solve_smem(rowsPerThread);
+        const cudaError_t e = once_per_device(done, [&] {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        });
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kCgCluster);
+        cfg.blockDim = dim3(kCgThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kCgCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        count_launch();
+        return cudaLaunchKernelEx(&cfg, kernel, m, rows, count, v, (const int32_t*)vs.slot_of, (const float*)vs.x,
+                                  (const double*)(fromX64 ? vs.x64 : nullptr), rel2, abs2, maxIter, iters);
+    };
+    static std::atomic<uint64_t> done[4];
+    const int per = (count + kCgCluster * kCgThreads - 1) / (kCgCluster * kCgThreads);
+    if (per <= 1) return go(k_cg_solve<1>, 1, done[0]);
+    if (per == 2) return go(k_cg_solve<2>, 2, done[1]);
+    if (per == 3) return go(k_cg_solve<3>, 3, done[2]);
+    return go(k_cg_solve<4>, 4, done[3]);
 }
 void launch_cg_replay_begin(int32_t* iter, double* tgt, double rel2, double abs2, cudaStream_t s) {
     count_launch();
