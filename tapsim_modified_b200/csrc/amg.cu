@@ -27,6 +27,7 @@ constexpr float kSmooth = kAmgSmooth;
 
 // y = w b / d
 __global__ void k_amg_jacobi(int n, const float* b, const float* d, float* y, Gate gate) {
+    chain_wait();
     if (gate.done()) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         y[i] = kSmooth * b[i] / d[i];
@@ -59,26 +60,49 @@ __device__ __forceinline__ void fine_last_round(const int* __restrict__ col, con
 #pragma unroll
     for (int j = 0; j < U; j++)
         if (k + j < width) {
-            acc += a[j] * __ldg(y + c[j]);
+            acc += a[j] * y[c[j]];
             sum += a[j];
         }
 }
 
 // U: the column/value loads a lane issues ahead of their gathers (the bytes
 // a warp keeps in flight), chosen per hierarchy by timed trials.
+// The first U couplings, which no kernel of the solve writes, load ahead of
+// the wait for the kernels before this one.
 template <int U>
 __global__ void k_amg_fine(VSys v, int slices, const float* b, const float* y, float* out, int mode, Gate gate) {
-    if (gate.done()) return;
     const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < slices; warp += warps) {
-        const int base = v.slice_start[warp];
-        const int width = v.slice_width[warp];
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int base = 0, width = 0;
+    if (warp < slices) {
+        base = v.slice_start[warp];
+        width = v.slice_width[warp];
+    }
+    const int* __restrict__ col = v.col + base + lane;
+    const __nv_bfloat16* __restrict__ val = v.val16 + base + lane;
+    int c0[U];
+    float a0[U];
+    if (width >= U) {
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+            c0[j] = __ldcs(col + 32 * j);
+            a0[j] = __bfloat162float(__ldcs(val + 32 * j));
+        }
+    }
+    chain_wait();
+    if (gate.done()) return;
+    if (warp < slices) {
         const int s = warp * 32 + lane;
-        const int* __restrict__ col = v.col + base + lane;
-        const __nv_bfloat16* __restrict__ val = v.val16 + base + lane;
         float acc = 0.0f, sum = 0.0f;
         int k = 0;
+        if (width >= U) {
+#pragma unroll
+            for (int j = 0; j < U; j++) {
+                acc += a0[j] * y[c0[j]];
+                sum += a0[j];
+            }
+            k = U;
+        }
         for (; k + U <= width; k += U) {
             int c[U];
             float a[U];
@@ -89,7 +113,7 @@ __global__ void k_amg_fine(VSys v, int slices, const float* b, const float* y, f
             }
 #pragma unroll
             for (int j = 0; j < U; j++) {
-                acc += a[j] * __ldg(y + c[j]);
+                acc += a[j] * y[c[j]];
                 sum += a[j];
             }
         }
@@ -107,6 +131,7 @@ __global__ void k_amg_fine(VSys v, int slices, const float* b, const float* y, f
 template <int U>
 __global__ void k_amg_fine_pipe(VSys v, int slices, const float* b, const float* y, float* out, int mode,
                                 Gate gate) {
+    chain_wait();
     if (gate.done()) return;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -140,7 +165,7 @@ __global__ void k_amg_fine_pipe(VSys v, int slices, const float* b, const float*
             }
 #pragma unroll
             for (int j = 0; j < U; j++) {
-                acc += a[j] * __ldg(y + c[j]);
+                acc += a[j] * y[c[j]];
                 sum += a[j];
             }
             if (more) {
@@ -164,27 +189,38 @@ __global__ void k_amg_fine_pipe(VSys v, int slices, const float* b, const float*
 // group for every row (no grid-stride loop, so that every row's loads are in
 // flight at once).  Each lane loads four of its entries before it gathers
 // their y, so that a row of up to 4 L entries costs one round trip.
+// The first four, like the row's bounds, load ahead of the wait for the
+// kernels before this one (no kernel of the solve writes the matrices).
 template <int L>
-__device__ __forceinline__ float row_dot(const int32_t* ptr, const int32_t* col, const float* val, const float* y,
-                                         int row, int lane) {
+__device__ __forceinline__ bool row_dot(const int32_t* ptr, const int32_t* col, const float* val, const float* y,
+                                        int row, int lane, const Gate& gate, float* out) {
     float acc = 0.0f;
     const int q1 = ptr[row + 1];
-    for (int q = ptr[row] + lane; q < q1; q += 4 * L) {
-        int c[4];
-        float a[4];
+    int q = ptr[row] + lane;
+    int c[4];
+    float a[4];
+    auto load = [&] {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const bool in = q + j * L < q1;
             c[j] = in ? __ldcs(col + q + j * L) : -1;
             a[j] = in ? __ldcs(val + q + j * L) : 0.0f;
         }
+    };
+    load();
+    chain_wait();
+    if (gate.done()) return false;
+    while (q < q1) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (c[j] >= 0) acc += a[j] * __ldg(y + c[j]);
+            if (c[j] >= 0) acc += a[j] * y[c[j]];
+        q += 4 * L;
+        load();
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    return acc;
+    *out = acc;
+    return true;
 }
 
 // Rows of a CSR operator A (with its diagonal):
@@ -192,11 +228,11 @@ __device__ __forceinline__ float row_dot(const int32_t* ptr, const int32_t* col,
 template <int L>
 __global__ void k_amg_csr(int n, const int32_t* ptr, const int32_t* col, const float* val, const float* diag,
                           const float* b, const float* y, float* out, int mode, Gate gate) {
-    if (gate.done()) return;
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = gid % L;
     const int row = min(gid / L, n - 1);  // whole groups stay active for the shuffles
-    const float acc = row_dot<L>(ptr, col, val, y, row, lane);
+    float acc;
+    if (!row_dot<L>(ptr, col, val, y, row, lane, gate, &acc)) return;
     if (lane == 0 && gid / L < n) {
         const float t = b[row] - acc;
         out[row] = mode == 0 ? t : y[row] + kSmooth * t / diag[row];
@@ -209,11 +245,11 @@ __global__ void k_amg_csr(int n, const int32_t* ptr, const int32_t* col, const f
 template <int L>
 __global__ void k_amg_mv(int n, const int32_t* ptr, const int32_t* col, const float* val, const float* y, float* out,
                          const float* diag, float* ysm, Gate gate) {
-    if (gate.done()) return;
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = gid % L;
     const int row = min(gid / L, n - 1);
-    const float acc = row_dot<L>(ptr, col, val, y, row, lane);
+    float acc;
+    if (!row_dot<L>(ptr, col, val, y, row, lane, gate, &acc)) return;
     if (lane == 0 && gid / L < n) {
         out[row] = acc;
         if (diag) ysm[row] = kSmooth * acc / diag[row];
@@ -223,16 +259,40 @@ __global__ void k_amg_mv(int n, const int32_t* ptr, const int32_t* col, const fl
 // y += P x' (prolongation, a few entries per row), one thread per row
 __global__ void k_amg_prolong(int n, const int32_t* ptr, const int32_t* col, const float* val, const float* xc,
                               float* y, Gate gate) {
+    // the first row's bounds and first entries ahead of the wait
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int q = 0, q1 = 0, c[4];
+    float a[4];
+    if (i < n) {
+        q = ptr[i];
+        q1 = ptr[i + 1];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const bool in = q + j < q1;
+        c[j] = in ? col[q + j] : -1;
+        a[j] = in ? val[q + j] : 0.0f;
+    }
+    chain_wait();
     if (gate.done()) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (i < n) {
         float acc = 0.0f;
-        for (int q = ptr[i]; q < ptr[i + 1]; q++) acc += val[q] * __ldg(xc + col[q]);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (c[j] >= 0) acc += a[j] * xc[c[j]];
+        for (q += 4; q < q1; q++) acc += val[q] * xc[col[q]];
+        y[i] += acc;
+    }
+    for (i += gridDim.x * blockDim.x; i < n; i += gridDim.x * blockDim.x) {
+        float acc = 0.0f;
+        for (int p = ptr[i]; p < ptr[i + 1]; p++) acc += val[p] * xc[col[p]];
         y[i] += acc;
     }
 }
 
 // x = C^-1 b with the coarsest level's dense inverse (row-major), one warp per row
 __global__ void k_amg_dense(int n, const float* inv, const float* b, float* x, Gate gate) {
+    chain_wait();
     if (gate.done()) return;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -255,11 +315,11 @@ void launch_fine(int U, const VSys& v, int slices, const float* b, const float* 
                  cudaStream_t s) {
     count_launch();
     const unsigned grid = grid_full((long long)slices * 32);
-    if (U == kFinePipe + 4) k_amg_fine_pipe<4><<<grid, kBlock, 0, s>>>(v, slices, b, y, out, mode, gate);
-    else if (U == kFinePipe + 8) k_amg_fine_pipe<8><<<grid, kBlock, 0, s>>>(v, slices, b, y, out, mode, gate);
-    else if (U == 4) k_amg_fine<4><<<grid, kBlock, 0, s>>>(v, slices, b, y, out, mode, gate);
-    else if (U == 16) k_amg_fine<16><<<grid, kBlock, 0, s>>>(v, slices, b, y, out, mode, gate);
-    else k_amg_fine<8><<<grid, kBlock, 0, s>>>(v, slices, b, y, out, mode, gate);
+    if (U == kFinePipe + 4) launch_chain(k_amg_fine_pipe<4>, grid, kBlock, s, v, slices, b, y, out, mode, gate);
+    else if (U == kFinePipe + 8) launch_chain(k_amg_fine_pipe<8>, grid, kBlock, s, v, slices, b, y, out, mode, gate);
+    else if (U == 4) launch_chain(k_amg_fine<4>, grid, kBlock, s, v, slices, b, y, out, mode, gate);
+    else if (U == 16) launch_chain(k_amg_fine<16>, grid, kBlock, s, v, slices, b, y, out, mode, gate);
+    else launch_chain(k_amg_fine<8>, grid, kBlock, s, v, slices, b, y, out, mode, gate);
 }
 
 // a group of L threads for every row
@@ -270,22 +330,22 @@ void launch_csr(int L, int n, const int32_t* ptr, const int32_t* col, const floa
                 const float* b, const float* y, float* out, int mode, Gate gate, cudaStream_t s) {
     count_launch();
     switch (L) {
-        case 2: k_amg_csr<2><<<grid_rows(n, 2), kBlock, 0, s>>>(n, ptr, col, val, diag, b, y, out, mode, gate); break;
-        case 4: k_amg_csr<4><<<grid_rows(n, 4), kBlock, 0, s>>>(n, ptr, col, val, diag, b, y, out, mode, gate); break;
-        case 8: k_amg_csr<8><<<grid_rows(n, 8), kBlock, 0, s>>>(n, ptr, col, val, diag, b, y, out, mode, gate); break;
-        case 16: k_amg_csr<16><<<grid_rows(n, 16), kBlock, 0, s>>>(n, ptr, col, val, diag, b, y, out, mode, gate); break;
-        default: k_amg_csr<32><<<grid_rows(n, 32), kBlock, 0, s>>>(n, ptr, col, val, diag, b, y, out, mode, gate); break;
+        case 2: launch_chain(k_amg_csr<2>, grid_rows(n, 2), kBlock, s, n, ptr, col, val, diag, b, y, out, mode, gate); break;
+        case 4: launch_chain(k_amg_csr<4>, grid_rows(n, 4), kBlock, s, n, ptr, col, val, diag, b, y, out, mode, gate); break;
+        case 8: launch_chain(k_amg_csr<8>, grid_rows(n, 8), kBlock, s, n, ptr, col, val, diag, b, y, out, mode, gate); break;
+        case 16: launch_chain(k_amg_csr<16>, grid_rows(n, 16), kBlock, s, n, ptr, col, val, diag, b, y, out, mode, gate); break;
+        default: launch_chain(k_amg_csr<32>, grid_rows(n, 32), kBlock, s, n, ptr, col, val, diag, b, y, out, mode, gate); break;
     }
 }
 void launch_mv(int L, int n, const int32_t* ptr, const int32_t* col, const float* val, const float* y, float* out,
                Gate gate, cudaStream_t s, const float* diag = nullptr, float* ysm = nullptr) {
     count_launch();
     switch (L) {
-        case 2: k_amg_mv<2><<<grid_rows(n, 2), kBlock, 0, s>>>(n, ptr, col, val, y, out, diag, ysm, gate); break;
-        case 4: k_amg_mv<4><<<grid_rows(n, 4), kBlock, 0, s>>>(n, ptr, col, val, y, out, diag, ysm, gate); break;
-        case 8: k_amg_mv<8><<<grid_rows(n, 8), kBlock, 0, s>>>(n, ptr, col, val, y, out, diag, ysm, gate); break;
-        case 16: k_amg_mv<16><<<grid_rows(n, 16), kBlock, 0, s>>>(n, ptr, col, val, y, out, diag, ysm, gate); break;
-        default: k_amg_mv<32><<<grid_rows(n, 32), kBlock, 0, s>>>(n, ptr, col, val, y, out, diag, ysm, gate); break;
+        case 2: launch_chain(k_amg_mv<2>, grid_rows(n, 2), kBlock, s, n, ptr, col, val, y, out, diag, ysm, gate); break;
+        case 4: launch_chain(k_amg_mv<4>, grid_rows(n, 4), kBlock, s, n, ptr, col, val, y, out, diag, ysm, gate); break;
+        case 8: launch_chain(k_amg_mv<8>, grid_rows(n, 8), kBlock, s, n, ptr, col, val, y, out, diag, ysm, gate); break;
+        case 16: launch_chain(k_amg_mv<16>, grid_rows(n, 16), kBlock, s, n, ptr, col, val, y, out, diag, ysm, gate); break;
+        default: launch_chain(k_amg_mv<32>, grid_rows(n, 32), kBlock, s, n, ptr, col, val, y, out, diag, ysm, gate); break;
     }
 }
 
@@ -397,7 +457,7 @@ void launch_amg_vcycle(const VSys& v, int slots, const AmgDev& g, int it, double
     const int slices = (slots + 31) / 32;
     if (!y0Ready) {
         count_launch();
-        k_amg_jacobi<<<grid_for(slots), kBlock, 0, s>>>(slots, v.r, v.d, g.y0, gate);
+        launch_chain(k_amg_jacobi, grid_for(slots), kBlock, s, slots, v.r, v.d, g.y0, gate);
     }
     if (g.levels > 1) {
         launch_fine(g.fine_unroll, v, slices, v.r, g.y0, g.t0, 0, gate, s);
@@ -409,7 +469,7 @@ void launch_amg_vcycle(const VSys& v, int slots, const AmgDev& g, int it, double
             if (l + 1 == g.levels - 1) {
                 launch_mv(L.r_lanes, C.n, L.r_ptr, L.r_col, L.r_val, t, C.b, gate, s);
                 count_launch();
-                k_amg_dense<<<grid_for((long long)C.n * 32), kBlock, 0, s>>>(C.n, g.coarse_inv, C.b, C.x, gate);
+                launch_chain(k_amg_dense, grid_for((long long)C.n * 32), kBlock, s, C.n, g.coarse_inv, C.b, C.x, gate);
             } else {
                 // the restriction also takes the coarse level's pre-smoothing step
                 launch_mv(L.r_lanes, C.n, L.r_ptr, L.r_col, L.r_val, t, C.b, gate, s, C.diag, C.y);
@@ -422,7 +482,7 @@ void launch_amg_vcycle(const VSys& v, int slots, const AmgDev& g, int it, double
             const AmgDevLevel& C = g.lev[l + 1];
             float* y = l == 0 ? g.y0 : L.y;
             count_launch();
-            k_amg_prolong<<<grid_for(L.n), kBlock, 0, s>>>(L.n, L.p_ptr, L.p_col, L.p_val, C.x, y, gate);
+            launch_chain(k_amg_prolong, grid_for(L.n), kBlock, s, L.n, L.p_ptr, L.p_col, L.p_val, C.x, y, gate);
             if (l == 0) {
                 launch_fine(g.fine_unroll, v, slices, v.r, g.y0, v.u, 1, gate, s);
             } else {

@@ -47,15 +47,18 @@ __device__ __forceinline__ void cg_coeffs(const double* scal, int it, double* al
 
 // x = 0, rho_0 = r.r; with the Jacobi preconditioner also u = r / d and
 // gamma_0 = r.u (with the multigrid one the V-cycle makes u and the SpMV
-// gamma)
-__global__ void k_vcg_init(VSys v, int slots, int jacobi) {
+// gamma; smoothY, when given, the V-cycle's first step)
+__global__ void k_vcg_init(VSys v, int slots, int jacobi, float* smoothY) {
     double g = 0.0, rr = 0.0;
+    chain_wait();
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < slots; s += gridDim.x * blockDim.x) {
         const float r = v.r[s];
         if (jacobi) {
             const float u = r / v.d[s];
             v.u[s] = u;
             g += (double)r * (double)u;
+        } else if (smoothY) {
+            smoothY[s] = kAmgSmooth * r / v.d[s];  // as k_amg_jacobi computes it
         }
         v.x[s] = 0.0f;
         v.p[s] = 0.0f;
@@ -69,23 +72,43 @@ __global__ void k_vcg_init(VSys v, int slots, int jacobi) {
 // u this is), and with withGamma gamma = r.u -> scal[4*it]; skipped once
 // iteration it has converged (cg_done)
 __global__ void k_vcg_spmv(VSys v, int slices, Gate gate, int withGamma) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // the slice's first couplings, which no kernel of the solve writes, ahead
+    // of the wait for the kernels before this one
+    int base = 0, width = 0;
+    if (warp < slices) {
+        base = v.slice_start[warp];
+        width = v.slice_width[warp];
+    }
+    const int* __restrict__ col = v.col + base + lane;
+    const float* __restrict__ val = v.val + base + lane;
+    int c0[8];
+    float a0[8];
+    if (width >= 8) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            c0[j] = __ldcs(col + 32 * j);
+            a0[j] = __ldcs(val + 32 * j);
+        }
+    }
+    chain_wait();
     if (gate.done()) return;
     const int it = gate.iter();
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
     double dl = 0.0, gl = 0.0;
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < slices; warp += warps) {
-        const int base = v.slice_start[warp];
-        const int width = v.slice_width[warp];
+    if (warp < slices) {
         const int s = warp * 32 + lane;
-        const int* __restrict__ col = v.col + base + lane;
-        const float* __restrict__ val = v.val + base + lane;
-        const float* __restrict__ uu = v.u;
+        const float* uu = v.u;
         float acc = 0.0f;
         // eight independent column/value loads ahead of their gathers keep
         // enough bytes in flight per warp; the matrix is streamed once per
         // iteration (evict-first), the gathered vector stays cached
         int k = 0;
+        if (width >= 8) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc += a0[j] * uu[c0[j]];
+            k = 8;
+        }
         for (; k + 8 <= width; k += 8) {
             int c[8];
             float a[8];
@@ -95,9 +118,9 @@ __global__ void k_vcg_spmv(VSys v, int slices, Gate gate, int withGamma) {
                 a[j] = __ldcs(val + 32 * (k + j));
             }
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc += a[j] * __ldg(uu + c[j]);
+            for (int j = 0; j < 8; j++) acc += a[j] * uu[c[j]];
         }
-        for (; k < width; k++) acc += __ldcs(val + 32 * k) * __ldg(uu + __ldcs(col + 32 * k));
+        for (; k < width; k++) acc += __ldcs(val + 32 * k) * uu[__ldcs(col + 32 * k)];
         const float u = v.u[s];
         const float w = v.d[s] * u - acc;
         v.w[s] = w;
@@ -114,6 +137,7 @@ __global__ void k_vcg_spmv(VSys v, int slices, Gate gate, int withGamma) {
 // gamma_{it+1} = r.u; with smoothY (the multigrid one) the V-cycle's first
 // step smoothY = w r / d, one launch fewer per iteration
 __global__ void k_vcg_update(VSys v, int slots, Gate gate, int jacobi, float* smoothY) {
+    chain_wait();
     if (gate.done()) return;
     const int it = gate.iter();
     double alpha, beta;
@@ -142,7 +166,10 @@ __global__ void k_vcg_update(VSys v, int slots, Gate gate, int jacobi, float* sm
 }
 
 // the replayed CG iterations' counter and target
-__global__ void k_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter) {
+// and, with scal, the accumulators of the start and of the first iteration
+__global__ void k_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter, double* scal) {
+    if (scal)
+        for (int k = 0; k < 8; k++) scal[k] = 0.0;
     *iter = 0;
     rel2Dev[0] = rel2;
     rel2Dev[1] = (double)maxIter;
@@ -154,10 +181,13 @@ __global__ void k_vcg_replay_step(int32_t* iter) { *iter += 1; }
 // loop goes on while fewer than the cap (rel2Dev[1]) have run and rho_k >
 // rel2 rho_0; a NaN stops it.  *done gets the iterations the solve took (0
 // when rho_0 is 0, as the host loop counts them).  The counter steps once per
-// pass, so the loop ends after the cap at the latest.
-__global__ void k_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, const double* scal,
+// pass, so the loop ends after the cap at the latest.  The next iteration's
+// accumulators start from zero.
+__global__ void k_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, double* scal,
                                 const double* rel2Dev, int32_t* done) {
+    chain_wait();
     const int k = *iter + 1;
+    for (int j = 0; j < 4; j++) scal[4 * (k + 1) + j] = 0.0;
     *iter = k;
     const double rho0 = scal[3];
     const bool more = k < (int)rel2Dev[1] && rho0 > 0.0 && scal[4 * k + 3] > rel2Dev[0] * rho0;
@@ -561,32 +591,35 @@ inline int reduce_blocks(int n) {
 
 }  // namespace
 
-void launch_vcg_init(const VSys& v, int slots, bool jacobi, cudaStream_t s) {
-    if (slots > 0) { count_launch(); k_vcg_init<<<reduce_blocks(slots), kBlock, 0, s>>>(v, slots, jacobi ? 1 : 0); }
+void launch_vcg_init(const VSys& v, int slots, bool jacobi, cudaStream_t s, float* smoothY) {
+    if (slots > 0) {
+        count_launch();
+        launch_chain(k_vcg_init, reduce_blocks(slots), kBlock, s, v, slots, jacobi ? 1 : 0, jacobi ? nullptr : smoothY);
+    }
 }
 void launch_vcg_spmv(const VSys& v, int slots, int it, double target, bool withGamma, cudaStream_t s) {
     const int slices = (slots + 31) / 32;
     if (slices > 0) {
         count_launch();
-        k_vcg_spmv<<<blocks(slices * 32), kBlock, 0, s>>>(v, slices, make_gate(v, it, target), withGamma ? 1 : 0);
+        launch_chain(k_vcg_spmv, blocks(slices * 32), kBlock, s, v, slices, make_gate(v, it, target), withGamma ? 1 : 0);
     }
 }
 void launch_vcg_update(const VSys& v, int slots, int it, double target, bool jacobi, cudaStream_t s,
                        float* smoothY) {
     if (slots > 0) {
         count_launch();
-        k_vcg_update<<<reduce_blocks(slots), kBlock, 0, s>>>(v, slots, make_gate(v, it, target), jacobi ? 1 : 0,
-                                                             jacobi ? nullptr : smoothY);
+        launch_chain(k_vcg_update, reduce_blocks(slots), kBlock, s, v, slots, make_gate(v, it, target), jacobi ? 1 : 0,
+                     jacobi ? nullptr : smoothY);
     }
 }
-void launch_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter, cudaStream_t s) {
+void launch_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter, cudaStream_t s, double* scal) {
     count_launch();
-    k_vcg_replay_begin<<<1, 1, 0, s>>>(iter, rel2Dev, rel2, maxIter);
+    k_vcg_replay_begin<<<1, 1, 0, s>>>(iter, rel2Dev, rel2, maxIter, scal);
 }
-void launch_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, const double* scal,
+void launch_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, double* scal,
                           const double* rel2Dev, int32_t* done, cudaStream_t s) {
     count_launch();
-    k_vcg_loop_cond<<<1, 1, 0, s>>>(loop, iter, scal, rel2Dev, done);
+    launch_chain(k_vcg_loop_cond, 1, 1, s, loop, iter, scal, rel2Dev, done);
 }
 void launch_vcg_replay_step(int32_t* iter, cudaStream_t s) {
     count_launch();

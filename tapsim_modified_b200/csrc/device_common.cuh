@@ -59,6 +59,15 @@ struct DType {
     uint8_t removable, neumann, dirichlet, present;
 };
 
+// Programmatic dependent launch (launch_chain below): a kernel of a chain
+// first loads what no kernel of the chain writes, then waits until the
+// kernels before it have completed; it lets the next kernel's blocks start as
+// soon as its own have.  Both are no-ops in a plain launch.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr double kEpsilon0 = 8.85418781762e-12;  // As/(Vm), grid_3d.h:283
 
 __device__ __forceinline__ void atomic_max_double_nonneg(double* addr, double v) {
@@ -146,6 +155,32 @@ __device__ __forceinline__ void block_max_atomic_u64(unsigned long long v, unsig
         if (lane == 0 && s != 0ull) atomicMax(out, s);
     }
     __syncthreads();
+}
+
+// Launches a kernel of a chain.  While a ChainScope lives on this thread, the
+// launch may overlap the end of the kernel before it in the stream (the
+// kernel calls chain_wait before it reads what the chain writes); otherwise
+// it is a plain launch.  Used in stream capture, where the chain's first
+// kernel follows the capture's start.
+inline thread_local bool t_chain = false;
+struct ChainScope {
+    ChainScope() { t_chain = true; }
+    ~ChainScope() { t_chain = false; }
+    ChainScope(const ChainScope&) = delete;
+    ChainScope& operator=(const ChainScope&) = delete;
+};
+template <class... P, class... A>
+inline void launch_chain(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = t_chain ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 // Runs f() (a cudaError_t-returning setup such as cudaFuncSetAttribute,

@@ -216,6 +216,7 @@ struct tg_handle {
     std::vector<uint64_t> loopKey;
     DBuf<int32_t> loopDone;              // [1] iterations of the last looped solve
     long long loopNodes = 0;             // kernels per iteration of the loop
+    long long loopStartNodes = 0;        // and of the solve's start before it
     std::vector<uint64_t> iterKey;       // the device state it was captured with
     long long iterNodes = 0;             // kernels in one replay
     // the same for the node-space CG iterations of either row list (run_cg)
@@ -1240,13 +1241,21 @@ static int iteration_graph(tg_handle* h, const VSys& vg) {
     return TG_OK;
 }
 
-// Launch mode 2: the replayed iteration inside a while-conditional graph
-// node.  The loop's body is the iteration (update, V-cycle, SpMV) and
-// k_vcg_loop_cond, which steps the device counter and sets the node's
-// condition from it and rho; the counter steps once per body, so the loop
-// ends by the iteration cap.  Captured anew with the iteration graph's key.
-static int iteration_loop_graph(tg_handle* h, const VSys& vg) {
-    std::vector<uint64_t> key = iteration_key(vg, h->amg, h->vActive);
+// Launch mode 2: the whole inner solve as one graph, its start (init, V-cycle,
+// SpMV) and then the replayed iteration inside a while-conditional node.  The
+// loop's body is the iteration (update, V-cycle, SpMV) and k_vcg_loop_cond,
+// which steps the device counter and sets the node's condition from it and
+// rho; the counter steps once per body, so the loop ends by the iteration
+// cap.  The kernels are chained (launch_chain): on a 307k-cell tip an
+// iteration is twelve kernels of a few us each, whose starts overlap the ends
+// of the ones before.  v: the VSys of the start (no counter); vg: the loop's.
+// slots: those in use, rounded up to kGraphSlots (the slots beyond hold
+// nothing, and their rows only zeros), so that removals seldom make it be
+// captured anew, which takes about 1.2 ms.
+constexpr int kGraphSlots = 1024;
+static int iteration_loop_graph(tg_handle* h, const VSys& v, const VSys& vg) {
+    const int slots = std::min(h->vCapacity, (h->vActive + kGraphSlots - 1) / kGraphSlots * kGraphSlots);
+    std::vector<uint64_t> key = iteration_key(vg, h->amg, slots);
     key.push_back((uint64_t)(uintptr_t)h->loopDone.p);
     if (h->loopExec && key == h->loopKey) return TG_OK;
     if (h->loopExec) {
@@ -1254,9 +1263,34 @@ static int iteration_loop_graph(tg_handle* h, const VSys& vg) {
         h->loopExec = nullptr;
     }
     if (!h->captureStream) CK(cudaStreamCreateWithFlags(&h->captureStream, cudaStreamNonBlocking));
-    const int slots = h->vActive;
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaGraphCreate(&graph, 0);
+    long long nodes = 0;
+    ChainScope chained;
+    t_captured = &nodes;
+    cudaError_t e = cudaStreamBeginCapture(h->captureStream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        cudaStream_t cs = h->captureStream;
+        launch_vcg_init(v, slots, false, cs, h->amg.y0);
+        launch_amg_vcycle(v, slots, h->amg, 0, -1.0, cs, true);
+        launch_vcg_spmv(v, slots, 0, -1.0, true, cs);
+        e = cudaStreamEndCapture(cs, &graph);
+    }
+    t_captured = nullptr;
+    h->loopStartNodes = nodes;  // kernels of the solve's start
+    nodes = 0;
+    // the loop follows the start's last kernel
+    cudaGraphNode_t last = nullptr;
+    if (e == cudaSuccess) {
+        size_t count = 0;
+        e = cudaGraphGetNodes(graph, nullptr, &count);
+        std::vector<cudaGraphNode_t> all(count);
+        if (e == cudaSuccess) e = cudaGraphGetNodes(graph, all.data(), &count);
+        for (size_t k = 0; e == cudaSuccess && k < count; k++) {
+            size_t followers = 0;
+            e = cudaGraphNodeGetDependentNodes_v2(all[k], nullptr, nullptr, &followers);
+            if (followers == 0) last = all[k];
+        }
+    }
     cudaGraphConditionalHandle loop{};
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&loop, graph, 1, cudaGraphCondAssignDefault);
     cudaGraphNodeParams params{};
@@ -1266,9 +1300,8 @@ static int iteration_loop_graph(tg_handle* h, const VSys& vg) {
         params.conditional.handle = loop;
         params.conditional.type = cudaGraphCondTypeWhile;
         params.conditional.size = 1;
-        e = cudaGraphAddNode(&node, graph, nullptr, 0, &params);
+        e = cudaGraphAddNode(&node, graph, &last, 1, &params);
     }
-    long long nodes = 0;
     if (e == cudaSuccess) {
         cudaGraph_t body = params.conditional.phGraph_out[0];
         t_captured = &nodes;
@@ -1543,20 +1576,37 @@ static int run_vcg(tg_handle* h, double rtol, int maxIter, bool amg, int* itersO
     if (h->vScal.n < need) CK(h->vScal.alloc(need));
     VSys v = h->vs();
     const int slots = h->vActive;
+    const double rel2 = rtol * rtol;
+    if (amg && !fp64 && h->launchMode == 2 && slots > 0) {
+        if (!h->iterDev.p) CK(h->iterDev.alloc(1));
+        if (!h->rel2Dev.p) CK(h->rel2Dev.alloc(2));
+        if (!h->loopDone.p) CK(h->loopDone.alloc(1));
+        VSys vg = v;
+        vg.iter = h->iterDev.p;
+        vg.rel2 = h->rel2Dev.p;
+        const int rc = iteration_loop_graph(h, v, vg);
+        if (rc != TG_OK) return rc;
+        launch_vcg_replay_begin(h->iterDev.p, h->rel2Dev.p, rel2, maxIter, h->stream, h->vScal.p);
+        // the whole solve in one launch: the loop stops itself
+        CK(cudaGraphLaunch(h->loopExec, h->stream));
+        g_launches.fetch_add(h->loopStartNodes, std::memory_order_relaxed);
+        CK(cudaMemcpyAsync(&h->pin->loopIters[0], h->loopDone.p, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        *itersOut = -1;  // pending: pin->loopIters[0] after the next sync
+        return TG_OK;
+    }
     CK(cudaMemsetAsync(h->vScal.p, 0, sizeof(double) * need, h->stream));
     if (fp64) {
         launch_vcg64_init(v, slots, h->resid.p, h->stream);
         launch_amg_vcycle(v, slots, h->amg, 0, -1.0, h->stream);
         launch_vcg64_spmv(v, slots, 0, -1.0, h->stream);
     } else {
-        launch_vcg_init(v, slots, !amg, h->stream);
-        if (amg) launch_amg_vcycle(v, slots, h->amg, 0, -1.0, h->stream);
+        launch_vcg_init(v, slots, !amg, h->stream, amg ? h->amg.y0 : nullptr);
+        if (amg) launch_amg_vcycle(v, slots, h->amg, 0, -1.0, h->stream, true);
         launch_vcg_spmv(v, slots, 0, -1.0, amg, h->stream);
     }
     // stop on the 2-norm of the residual (rho = r.r), the norm the outer
     // FP64 test uses: rho_it <= rtol^2 rho_0, tested by the kernels
     // themselves, so the iterations queue before rho_0 is read back
-    const double rel2 = rtol * rtol;
     // the multigrid FP32 iterations replay one captured iteration
     const bool replay = amg && !fp64 && h->launchMode >= 1 && slots > 0;
     if (replay) {
@@ -1565,18 +1615,9 @@ static int run_vcg(tg_handle* h, double rtol, int maxIter, bool amg, int* itersO
         VSys vg = v;
         vg.iter = h->iterDev.p;
         vg.rel2 = h->rel2Dev.p;
-        if (h->launchMode == 2 && !h->loopDone.p) CK(h->loopDone.alloc(1));
-        const int rc = h->launchMode == 2 ? iteration_loop_graph(h, vg) : iteration_graph(h, vg);
+        const int rc = iteration_graph(h, vg);
         if (rc != TG_OK) return rc;
         launch_vcg_replay_begin(h->iterDev.p, h->rel2Dev.p, rel2, maxIter, h->stream);
-        if (h->launchMode == 2) {
-            // the whole solve in one launch: the loop stops itself
-            CK(cudaGraphLaunch(h->loopExec, h->stream));
-            CK(cudaMemcpyAsync(&h->pin->loopIters[0], h->loopDone.p, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                               h->stream));
-            *itersOut = -1;  // pending: pin->loopIters[0] after the next sync
-            return TG_OK;
-        }
     }
     int it = 0;
     // iterations queued before the first read: about as many as the last

@@ -133,7 +133,8 @@ inline Gate open_gate() { return Gate{nullptr, 0, -1.0, nullptr, nullptr}; }
 // otherwise u comes from launch_amg_vcycle and the SpMV adds gamma = r.u.
 // `target` of the iteration kernels (and of the V-cycle) is relative: they
 // do nothing once rho_it <= target * rho_0; a negative target never skips
-void launch_vcg_init(const VSys& v, int slots, bool jacobi, cudaStream_t s);
+// smoothY (multigrid preconditioner): as launch_vcg_update's
+void launch_vcg_init(const VSys& v, int slots, bool jacobi, cudaStream_t s, float* smoothY = nullptr);
 void launch_vcg_spmv(const VSys& v, int slots, int it, double target, bool withGamma, cudaStream_t s);
 // smoothY (multigrid preconditioner): also the V-cycle's first step,
 // smoothY = kAmgSmooth r / d, so that the cycle that follows skips it
@@ -142,11 +143,13 @@ void launch_vcg_update(const VSys& v, int slots, int it, double target, bool jac
 // the counter, target and cap of iterations replayed from a CUDA graph:
 // set to 0, rel2 and maxIter before the first replay, stepped by 1 at the
 // end of each
-void launch_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter, cudaStream_t s);
+// scal (may be null): the accumulators to clear for a looped solve
+void launch_vcg_replay_begin(int32_t* iter, double* rel2Dev, double rel2, int maxIter, cudaStream_t s,
+                             double* scal = nullptr);
 // the condition kernel of the device-side loop around the replayed
 // iteration (the last node of the loop's body): steps *iter, then sets the
 // loop's condition; *done: the iterations run
-void launch_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, const double* scal,
+void launch_vcg_loop_cond(cudaGraphConditionalHandle loop, int32_t* iter, double* scal,
                           const double* rel2Dev, int32_t* done, cudaStream_t s);
 void launch_vcg_replay_step(int32_t* iter, cudaStream_t s);
 // FP64 inner iterations with the multigrid preconditioner: the V-cycle runs
