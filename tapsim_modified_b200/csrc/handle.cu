@@ -464,26 +464,27 @@ int refresh_counts(tg_handle* h) {
     return TG_OK;
 }
 
-int ensure_bnorm(tg_handle* h) {
-    if (h->bnormValid) return TG_OK;
+// n coloured sweeps over all free rows; devAcc receives max |delta| of the
+// last.  All but the first launch are links of a chain: none of them writes
+// what the next loads before it waits
+void sweep_all(tg_handle* h, int32_t n, double* devAcc) {
     DevMesh m = h->dm();
-    CK(cudaMemsetAsync(h->acc.p, 0, sizeof(double), h->stream));
-    launch_bnorm(m, h->allV.p, h->countAllV, h->acc.p, h->stream);
-    launch_bnorm(m, h->allN.p, h->countAllN, h->acc.p, h->stream);
-    CK(cudaMemcpyAsync(&h->bnorm2, h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    const int rc = sync_status(h, "bnorm");
-    if (rc != TG_OK) return rc;
-    h->bnormValid = true;
-    return TG_OK;
-}
-
-// one coloured sweep over all free rows; dev receives max |delta| when non-null
-void sweep_all(tg_handle* h, double* devAcc) {
-    DevMesh m = h->dm();
-    for (int c = 0; c < h->ncol; c++) {
-        launch_sweep64(m, h->rowsV.p + h->segStart[c], h->countV[c], devAcc, h->stream);
-        launch_sweep64(m, h->rowsN.p + h->segStart[c], h->countN[c], devAcc, h->stream);
-    }
+    bool first = true;
+    for (int32_t it = 0; it < n; it++)
+        for (int c = 0; c < h->ncol; c++) {
+            if (h->countV[c] + h->countN[c] <= 0) continue;
+            auto go = [&] {
+                launch_sweep64(m, h->rowsV.p + h->segStart[c], h->countV[c], h->rowsN.p + h->segStart[c], h->countN[c],
+                               it == n - 1 ? devAcc : nullptr, h->stream);
+            };
+            if (first) {
+                go();
+            } else {
+                ChainScope chained;
+                go();
+            }
+            first = false;
+        }
 }
 
 // regression slope of the deviation queue as Grid_3d::Table::relax computes
@@ -1062,13 +1063,11 @@ int tg_get_types(tg_handle* h, int8_t* out) {
 int tg_relax_cycles(tg_handle* h, int32_t n, double* deviation) {
     DeviceScope dev_scope(h);
     if (!h || n < 1) return fail(h, TG_ERR_ARGUMENT, "tg_relax_cycles: bad argument");
-    for (int it = 0; it < n - 1; it++) sweep_all(h, nullptr);
     CK(cudaMemsetAsync(h->acc.p, 0, sizeof(double), h->stream));
-    sweep_all(h, h->acc.p);
-    double dev = 0.0;
-    CK(cudaMemcpyAsync(&dev, h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    sweep_all(h, n, h->acc.p);
+    CK(cudaMemcpyAsync(&h->pin->sums[2], h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     const int rc = sync_status(h, "tg_relax_cycles");
-    if (deviation) *deviation = dev;
+    if (deviation) *deviation = h->pin->sums[2];
     h->selValid = false;
     h->converged = h->histValid = h->residValid = false;
     return rc;
@@ -1110,26 +1109,16 @@ int tg_local_relax(tg_handle* h, int32_t node, int32_t shell, double threshold, 
     DevMesh m = h->dm();
     launch_local_set(m, node, shell, h->local.p, h->localCount.p, (int)h->local.n, h->localScratch.p,
                      (int)h->localScratch.n, h->ncol, h->stream);
-    std::vector<int32_t> counts(h->ncol + 2);
-    CK(cudaMemcpyAsync(counts.data(), h->localCount.p, sizeof(int32_t) * (h->ncol + 2), cudaMemcpyDeviceToHost,
-                       h->stream));
-    int rc = sync_status(h, "tg_local_relax");
-    if (rc != TG_OK) return rc;
-    std::vector<int32_t> offs(h->ncol, 0);
-    for (int c = 1; c < h->ncol; c++) offs[c] = offs[c - 1] + counts[c - 1];
+    int rc = TG_OK;
     std::deque<double> queue;
     int64_t iter = 0;
     double dev = 0.0;
     do {
-        for (int it = 0; it < cycle; it++) {
-            const bool last = it == cycle - 1;
-            if (last) CK(cudaMemsetAsync(h->acc.p, 0, sizeof(double), h->stream));
-            for (int c = 0; c < h->ncol; c++)
-                launch_sweep64(m, h->local.p + offs[c], counts[c], last ? h->acc.p : nullptr, h->stream);
-        }
-        CK(cudaMemcpyAsync(&dev, h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        launch_local_sweeps(m, h->local.p, h->localCount.p, h->ncol, cycle, h->acc.p, h->stream);
+        CK(cudaMemcpyAsync(&h->pin->sums[2], h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         rc = sync_status(h, "tg_local_relax");
         if (rc != TG_OK) break;
+        dev = h->pin->sums[2];
         queue.push_back(dev);
         while ((int)queue.size() > queueSize) queue.pop_front();
         if (stagnated(queue, (unsigned)queueSize, (unsigned)cycle)) {
@@ -1151,15 +1140,20 @@ int tg_local_relax(tg_handle* h, int32_t node, int32_t shell, double threshold, 
 int tg_residual(tg_handle* h, double* rel) {
     DeviceScope dev_scope(h);
     if (!h || !rel) return fail(h, TG_ERR_ARGUMENT, "tg_residual: null argument");
-    int rc = ensure_bnorm(h);
-    if (rc != TG_OK) return rc;
+    // ||b||^2 comes with the residual's pass when it is not known
     DevMesh m = h->dm();
-    CK(cudaMemsetAsync(h->acc.p, 0, sizeof(double), h->stream));
-    launch_residual(m, h->allV.p, h->countAllV, nullptr, h->acc.p, h->stream);
-    launch_residual(m, h->allN.p, h->countAllN, nullptr, h->acc.p, h->stream);
-    double r2 = 0.0;
-    CK(cudaMemcpyAsync(&r2, h->acc.p, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    rc = sync_status(h, "tg_residual");
+    double* bacc = h->bnormValid ? nullptr : h->acc.p + 1;
+    CK(cudaMemsetAsync(h->acc.p, 0, 2 * sizeof(double), h->stream));
+    launch_residual(m, h->allV.p, h->countAllV, nullptr, h->acc.p, h->stream, bacc);
+    launch_residual(m, h->allN.p, h->countAllN, nullptr, h->acc.p, h->stream, bacc);
+    CK(cudaMemcpyAsync(h->pin->sums + 2, h->acc.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    const int rc = sync_status(h, "tg_residual");
+    if (rc != TG_OK) return rc;
+    const double r2 = h->pin->sums[2];
+    if (bacc) {
+        h->bnorm2 = h->pin->sums[3];
+        h->bnormValid = true;
+    }
     *rel = h->bnorm2 > 0.0 ? std::sqrt(r2 / h->bnorm2) : std::sqrt(r2);
     return rc;
 }

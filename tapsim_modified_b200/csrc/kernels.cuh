@@ -232,18 +232,22 @@ void launch_vsys_refresh(const DevMesh& m, const VSys& v, const int32_t* nodes, 
 void launch_vsys_derive(const VSys& v, size_t stored, cudaStream_t s);
 
 // ---- relaxation (relax.cu) ----
-// coloured Gauss-Seidel sweep of one row list, FP64, max |delta| to *maxdev
-void launch_sweep64(const DevMesh& m, const int32_t* rows, int count, double* maxdev, cudaStream_t s);
+// one colour of a Gauss-Seidel sweep, FP64: its non-Neumann and Neumann rows;
+// max |delta| to *maxdev (may be null).  A link of a chain
+void launch_sweep64(const DevMesh& m, const int32_t* rowsV, int countV, const int32_t* rowsN, int countN,
+                    double* maxdev, cudaStream_t s);
+// whole sweeps over the set of launch_local_set (its rows and counts), max
+// |delta| of the last one to *maxdev
+void launch_local_sweeps(const DevMesh& m, const int32_t* rows, const int32_t* counts, int ncolours, int sweeps,
+                         double* maxdev, cudaStream_t s);
 // r_i (FP64) for a row list; accumulates sum r^2 into *acc; optionally
 // stores r as float into r32
-// with bacc, also the squared norm of the rows' Dirichlet part (as
-// launch_bnorm) into *bacc
+// with bacc, also the squared norm of the rows' Dirichlet part b_i = sum over
+// Dirichlet neighbours ceff_ij phi_j - q_i into *bacc
 // slotOf (may be null): r32 is indexed by slotOf[i] instead of i
 void launch_residual(const DevMesh& m, const int32_t* rows, int count, float* r32, double* acc, cudaStream_t s,
                      double* bacc = nullptr, double* r64 = nullptr, double* b64 = nullptr,
                      const int32_t* slotOf = nullptr);
-// b_i = sum over Dirichlet neighbours c_ij phi_j - q_i; sum b^2 into *acc
-void launch_bnorm(const DevMesh& m, const int32_t* rows, int count, double* acc, cudaStream_t s);
 // FP32 conjugate gradients on the rows of one list (Jacobi preconditioner)
 struct CGVectors {
     float *x, *r, *z, *p, *ap;

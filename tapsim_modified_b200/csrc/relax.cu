@@ -21,34 +21,101 @@ namespace {
 
 constexpr int kBlock = 256;
 
-__global__ void k_sweep64(DevMesh m, const int32_t* __restrict__ rows, int count, double* maxdev) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double dev = 0.0;
-    if (t < count) {
-        const int i = rows[t];
-        const int q0 = m.row_ptr[i], q1 = m.row_ptr[i + 1];
-        double s = 0.0;
-        for (int q = q0; q < q1; q++) s += m.ceff64[q] * m.phi64[m.col[q]];
-        const double d = m.diag64[i];
-        const double v = (s - m.q64[i]) / d;
-        if (!(v == v)) {
-            atomicOr(m.status, S_NAN);
-        } else {
-            dev = fabs(v - m.phi64[i]);
-            m.phi64[i] = v;
-        }
+// One row's update: phi_i = (sum_j ceff_ij phi_j - q_i) / diag_i, the sum in
+// CSR order; returns |delta|, 0 with S_NAN for a NaN.  Row holds what no
+// sweep writes, the first kAhead couplings among it, so that a thread has it
+// in registers before the sweep before its own has ended, and the row costs
+// one round of gathers.
+struct SweepRow {
+    static constexpr int kAhead = 16;
+    int i, q0, q1;
+    double d, qi;
+    int c[kAhead];
+    double a[kAhead];
+};
+__device__ __forceinline__ void sweep_load(const DevMesh& m, int i, SweepRow& r) {
+    r.i = i;
+    r.q0 = m.row_ptr[i];
+    r.q1 = m.row_ptr[i + 1];
+    r.d = m.diag64[i];
+    r.qi = m.q64[i];
+#pragma unroll
+    for (int k = 0; k < SweepRow::kAhead; k++) {
+        const bool in = r.q0 + k < r.q1;
+        r.c[k] = in ? m.col[r.q0 + k] : i;
+        r.a[k] = in ? m.ceff64[r.q0 + k] : 0.0;
     }
+}
+__device__ __forceinline__ double sweep_row(const DevMesh& m, const SweepRow& r) {
+    double p[SweepRow::kAhead];
+#pragma unroll
+    for (int k = 0; k < SweepRow::kAhead; k++) p[k] = m.phi64[r.c[k]];
+    const double old = m.phi64[r.i];
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < SweepRow::kAhead; k++)
+        if (r.q0 + k < r.q1) s = fma(r.a[k], p[k], s);
+    for (int q = r.q0 + SweepRow::kAhead; q < r.q1; q++) s = fma(m.ceff64[q], m.phi64[m.col[q]], s);
+    const double v = (s - r.qi) / r.d;
+    if (!(v == v)) {
+        atomicOr(m.status, S_NAN);
+        return 0.0;
+    }
+    m.phi64[r.i] = v;
+    return fabs(v - old);
+}
+
+// One colour of a sweep over all free cells, the non-Neumann and the Neumann
+// rows together (cells of one colour are never neighbours, so their order
+// does not matter).  A colour of a 307k-cell tip is 15k rows, a microsecond's
+// work: small blocks put it on every SM, and as links of a chain
+// (launch_chain) the colours follow one another without a launch's gap.
+// Separate launches of a thread per row that loaded as it went took 193 us a
+// sweep there, these 48.
+constexpr int kSweepBlock = 64;
+__global__ void __launch_bounds__(kSweepBlock) k_sweep64(DevMesh m, const int32_t* __restrict__ rowsV, int countV,
+                                                         const int32_t* __restrict__ rowsN, int countN,
+                                                         double* maxdev) {
+    const int t = blockIdx.x * kSweepBlock + threadIdx.x;
+    const bool live = t < countV + countN;
+    SweepRow r;
+    if (live) sweep_load(m, t < countV ? rowsV[t] : rowsN[t - countV], r);
+    chain_wait();
+    double dev = live ? sweep_row(m, r) : 0.0;
     if (maxdev) {
-        __shared__ double red[kBlock / 32];
         dev = warp_max_d(dev);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dev;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            double v = threadIdx.x < kBlock / 32 ? red[threadIdx.x] : 0.0;
-            v = warp_max_d(v);
-            if (threadIdx.x == 0 && v > 0.0) atomic_max_double_nonneg(maxdev, v);
+        if ((threadIdx.x & 31) == 0 && dev > 0.0) atomic_max_double_nonneg(maxdev, dev);
+    }
+}
+
+// `sweeps` sweeps over the rows that k_local_set has grouped by colour, one
+// block; max |delta| of the last sweep into *maxdev (cleared first).  A shell
+// is a few hundred cells: a barrier per colour in one block costs less than
+// a launch per colour.
+constexpr int kLocalThreads = 512;
+__global__ void __launch_bounds__(kLocalThreads) k_local_sweeps(DevMesh m, const int32_t* __restrict__ rows,
+                                                                const int32_t* __restrict__ counts, int ncolours,
+                                                                int sweeps, double* maxdev) {
+    if (threadIdx.x == 0) *maxdev = 0.0;
+    double dev = 0.0;
+    for (int it = 0; it < sweeps; it++) {
+        dev = 0.0;
+        int first = 0;
+        for (int c = 0; c < ncolours; c++) {
+            const int n = counts[c];
+            if (n == 0) continue;
+            for (int t = threadIdx.x; t < n; t += kLocalThreads) {
+                SweepRow r;
+                sweep_load(m, rows[first + t], r);
+                dev = fmax(dev, sweep_row(m, r));
+            }
+            first += n;
+            __syncthreads();
         }
     }
+    __syncthreads();
+    dev = warp_max_d(dev);
+    if ((threadIdx.x & 31) == 0 && dev > 0.0) atomic_max_double_nonneg(maxdev, dev);
 }
 
 // FP64 residual r_i = sum_j ceff_ij phi_j - diag_i phi_i - q_i of a row
@@ -62,7 +129,7 @@ __global__ void k_sweep64(DevMesh m, const int32_t* __restrict__ rows, int count
 // V system's slot) and at i otherwise; r64 and b64 (may be null) keep r and
 // the Dirichlet part by node.  With bacc, also the squared norm of the rows'
 // Dirichlet part b_i = sum over Dirichlet neighbours ceff_ij phi_j - q_i
-// (k_bnorm's value) from the same pass.
+// from the same pass.
 __global__ void k_residual(DevMesh m, const int32_t* __restrict__ rows, int count, float* r32,
                            const int32_t* __restrict__ slotOf, double* acc, double* bacc, double* r64, double* b64) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -89,22 +156,6 @@ __global__ void k_residual(DevMesh m, const int32_t* __restrict__ rows, int coun
     }
     if (withB) block_sum2_atomic<kBlock>(r2, b2, acc, bacc);
     else block_sum_atomic<kBlock>(r2, acc);
-}
-
-__global__ void k_bnorm(DevMesh m, const int32_t* __restrict__ rows, int count, double* acc) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double b = 0.0;
-    if (t < count) {
-        const int i = rows[t];
-        const int q0 = m.row_ptr[i], q1 = m.row_ptr[i + 1];
-        double s = 0.0;
-        for (int q = q0; q < q1; q++) {
-            const int j = m.col[q];
-            if (m.flags[j] & F_DIRICHLET) s += m.ceff64[q] * m.phi64[j];
-        }
-        b = s - m.q64[i];
-    }
-    block_sum_atomic<kBlock>(b * b, acc);
 }
 
 // z = r / diag, p = z, rz -> scal[0]
@@ -533,8 +584,18 @@ inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
 
 }  // namespace
 
-void launch_sweep64(const DevMesh& m, const int32_t* rows, int count, double* maxdev, cudaStream_t s) {
-    if (count > 0) { count_launch(); k_sweep64<<<blocks(count), kBlock, 0, s>>>(m, rows, count, maxdev); }
+void launch_sweep64(const DevMesh& m, const int32_t* rowsV, int countV, const int32_t* rowsN, int countN,
+                    double* maxdev, cudaStream_t s) {
+    const int rows = countV + countN;
+    if (rows <= 0) return;
+    count_launch();
+    launch_chain(k_sweep64, (unsigned)((rows + kSweepBlock - 1) / kSweepBlock), kSweepBlock, s, m, rowsV, countV, rowsN,
+                 countN, maxdev);
+}
+void launch_local_sweeps(const DevMesh& m, const int32_t* rows, const int32_t* counts, int ncolours, int sweeps,
+                         double* maxdev, cudaStream_t s) {
+    count_launch();
+    k_local_sweeps<<<1, kLocalThreads, 0, s>>>(m, rows, counts, ncolours, sweeps, maxdev);
 }
 void launch_residual(const DevMesh& m, const int32_t* rows, int count, float* r32, double* acc, cudaStream_t s,
                      double* bacc, double* r64, double* b64, const int32_t* slotOf) {
@@ -542,9 +603,6 @@ void launch_residual(const DevMesh& m, const int32_t* rows, int count, float* r3
     count_launch();
     b64 = bacc ? b64 : nullptr;
     k_residual<<<blocks(count), kBlock, 0, s>>>(m, rows, count, r32, slotOf, acc, bacc, r64, b64);
-}
-void launch_bnorm(const DevMesh& m, const int32_t* rows, int count, double* acc, cudaStream_t s) {
-    if (count > 0) { count_launch(); k_bnorm<<<blocks(count), kBlock, 0, s>>>(m, rows, count, acc); }
 }
 void launch_cg_init(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s) {
     if (count > 0) { count_launch(); k_cg_init<<<blocks(count), kBlock, 0, s>>>(m, rows, count, v); }
