@@ -402,6 +402,9 @@ void launch_apply_prediction(const DevMesh& m, const int32_t* nodes, const int32
                              cudaStream_t s);
 void launch_collect_target(const DevMesh& m, const int32_t* nodes, const int32_t* count, const double* phiStart,
                            const float* scale, float* tgt, int cap, cudaStream_t s);
-void launch_shift_cols(int32_t* col, int count, int shift, cudaStream_t s);
+// a training batch gathered from the sample store (table: k_stage_batch)
+void launch_stage_batch(const int64_t* table, int batch, int rows, int D, const float* sX, const float* sW,
+                        const int32_t* sCol, const float* sT, float* bX, float* bW, int32_t* bCol, float* bT,
+                        cudaStream_t s);
 
 }  // namespace tgd

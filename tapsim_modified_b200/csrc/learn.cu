@@ -97,6 +97,7 @@ struct tg_learner {
     // batch staging
     Buf<float> bX, bW, bT;
     Buf<int32_t> bCol;
+    Buf<int64_t> table;  // of the batches being staged (launch_stage_batch)
     // samples: concatenated per-cell data, host index
     Buf<float> sX, sW, sT;
     Buf<int32_t> sCol;
@@ -198,13 +199,13 @@ int forward(tg_learner* L, const float* X, const int32_t* col, const float* w, i
     return TG_OK;
 }
 
-// Loss and gradients (into L->G) of the rows forwarded last, against tgt
-int backward(tg_learner* L, const int32_t* col, const float* w, const float* tgt, int n, float* lossOut) {
+// Loss (added to *lossDev) and gradients (into L->G) of the rows forwarded
+// last, against tgt
+int backward(tg_learner* L, const int32_t* col, const float* w, const float* tgt, int n, float* lossDev) {
     const int npad = roundup128(std::max(n, 1));
     cudaStream_t s = L->stream;
     LCK(cudaMemsetAsync(L->G.p, 0, sizeof(float) * kParams, s));
-    LCK(cudaMemsetAsync(L->loss.p, 0, sizeof(float), s));
-    launch_loss(L->y.p, tgt, n, 1.0f / (float)std::max(n, 1), L->dy.p, L->loss.p, s);
+    launch_loss(L->y.p, tgt, n, 1.0f / (float)std::max(n, 1), L->dy.p, lossDev, s);
     launch_readout_back(L->Hl(kLayers - 1), L->dy.p, L->wout(), n, npad, L->gWl(kLayers) /* w_out */,
                         L->gWl(kLayers) + kHid /* b_out */, L->dH.p, s);
     int rc;
@@ -220,34 +221,45 @@ int backward(tg_learner* L, const int32_t* col, const float* w, const float* tgt
         std::swap(L->dH.p, L->dHp.p);
     }
     LCK(cudaGetLastError());
-    if (lossOut) LCK(cudaMemcpyAsync(lossOut, L->loss.p, sizeof(float), cudaMemcpyDeviceToHost, s));
     return TG_OK;
 }
 
-// Copies samples `idx` into the batch staging buffers; returns the rows
-int stage_batch(tg_learner* L, const std::vector<int>& idx, int* rowsOut) {
-    int64_t rows = 0;
-    for (int k : idx) rows += L->sLen[k];
-    if (rows > (1 << 22)) return lfail(L, TG_ERR_ARGUMENT, "learner: batch too large");
-    int rc = ensure_rows(L, roundup128((int)std::max<int64_t>(rows, 1)));
-    if (rc != TG_OK) return rc;
-    cudaStream_t s = L->stream;
-    int64_t at = 0;
-    for (int k : idx) {
-        const int64_t o = L->sOff[k];
-        const int len = L->sLen[k];
-        LCK(cudaMemcpyAsync(L->bX.p + at * kFeat, L->sX.p + o * kFeat, sizeof(float) * len * kFeat,
-                            cudaMemcpyDeviceToDevice, s));
-        LCK(cudaMemcpyAsync(L->bW.p + at * L->D, L->sW.p + o * L->D, sizeof(float) * len * L->D,
-                            cudaMemcpyDeviceToDevice, s));
-        LCK(cudaMemcpyAsync(L->bCol.p + at * L->D, L->sCol.p + o * L->D, sizeof(int32_t) * len * L->D,
-                            cudaMemcpyDeviceToDevice, s));
-        LCK(cudaMemcpyAsync(L->bT.p + at, L->sT.p + o, sizeof(float) * len, cudaMemcpyDeviceToDevice, s));
-        launch_shift_cols(L->bCol.p + at * L->D, len * L->D, (int)at, s);
-        at += len;
+// The tables of batches of samples (idx: the batches' samples in turn) onto
+// the device, their rows (rowsOut, one per batch), the staging buffers sized
+// for the largest and a zeroed loss for each
+int stage_tables(tg_learner* L, const std::vector<int>& idx, int batch, std::vector<int>* rowsOut) {
+    const size_t batches = idx.size() / batch, words = 2 * (size_t)batch + 1;
+    std::vector<int64_t> table(batches * words);
+    int64_t most = 1;
+    rowsOut->clear();
+    for (size_t s = 0; s < batches; s++) {
+        int64_t* off = table.data() + s * words;
+        int64_t at = 0;
+        for (int b = 0; b < batch; b++) {
+            const int k = idx[s * batch + b];
+            off[b] = L->sOff[k];
+            off[batch + b] = at;
+            at += L->sLen[k];
+        }
+        off[2 * batch] = at;
+        if (at > (1 << 22)) return lfail(L, TG_ERR_ARGUMENT, "learner: batch too large");
+        most = std::max(most, at);
+        rowsOut->push_back((int)at);
     }
-    *rowsOut = (int)rows;
+    const int rc = ensure_rows(L, roundup128((int)most));
+    if (rc != TG_OK) return rc;
+    if (L->table.n < table.size()) LCK(L->table.alloc(table.size()));
+    if (L->loss.n < batches) LCK(L->loss.alloc(batches));
+    LCK(cudaMemcpyAsync(L->table.p, table.data(), sizeof(int64_t) * table.size(), cudaMemcpyHostToDevice, L->stream));
+    LCK(cudaMemsetAsync(L->loss.p, 0, sizeof(float) * std::max<size_t>(batches, 1), L->stream));
+    LCK(cudaStreamSynchronize(L->stream));  // the table's host copy ends here
     return TG_OK;
+}
+
+// Gathers batch s of the staged tables (its rows: rows)
+void stage_batch(tg_learner* L, int s, int batch, int rows) {
+    launch_stage_batch(L->table.p + (size_t)s * (2 * (size_t)batch + 1), batch, rows, L->D, L->sX.p, L->sW.p, L->sCol.p,
+                       L->sT.p, L->bX.p, L->bW.p, L->bCol.p, L->bT.p, L->stream);
 }
 
 // Builds the graph of `site` from the current state on stream s; with nOut
@@ -423,7 +435,7 @@ void tg_learner_destroy(tg_learner* L) {
     L->scale.release(); L->X.release(); L->ellW.release(); L->ellCol.release(); L->phiStart.release();
     L->Z.release(); L->ZT.release(); L->DU.release(); L->DUT.release(); L->U.release(); L->H.release();
     L->C.release(); L->y.release(); L->dy.release(); L->dH.release(); L->dHp.release();
-    L->loss.release(); L->bX.release(); L->bW.release(); L->bT.release(); L->bCol.release();
+    L->loss.release(); L->table.release(); L->bX.release(); L->bW.release(); L->bT.release(); L->bCol.release();
     L->sX.release(); L->sW.release(); L->sT.release(); L->sCol.release();
     if (L->stream) cudaStreamDestroy(L->stream);
     delete L;
@@ -495,14 +507,16 @@ int tg_learner_gradients(tg_learner* L, int32_t first, int32_t count, float* los
         return lfail(L, TG_ERR_ARGUMENT, "tg_learner_gradients: bad sample range");
     std::vector<int> idx;
     for (int k = first; k < first + count; k++) idx.push_back(k);
-    int rows = 0;
-    int rc = stage_batch(L, idx, &rows);
-    if (rc == TG_OK) rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows);
-    float l = 0.0f;
-    if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows, &l);
+    std::vector<int> rowsOf;
+    int rc = stage_tables(L, idx, count, &rowsOf);
+    if (rc != TG_OK) return rc;
+    const int rows = rowsOf[0];
+    stage_batch(L, 0, count, rows);
+    rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows);
+    if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows, L->loss.p);
     if (rc == TG_OK) rc = check_status(L, "tg_learner_gradients");
     if (rc != TG_OK) return rc;
-    if (loss) *loss = l;
+    if (loss) LCK(cudaMemcpy(loss, L->loss.p, sizeof(float), cudaMemcpyDeviceToHost));
     if (grads) LCK(cudaMemcpy(grads, L->G.p, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
     if (outputs) LCK(cudaMemcpy(outputs, L->y.p, sizeof(float) * rows, cudaMemcpyDeviceToHost));
     return TG_OK;
@@ -519,13 +533,16 @@ int tg_learner_train(tg_learner* L, int32_t steps, int32_t batch, float lr, uint
     std::uniform_int_distribution<int> pick(first, first + count - 1);
     std::vector<float> losses(steps, 0.0f);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    // every step's samples drawn and their tables sent ahead, the losses read
+    // at the end, so that the steps queue without the host
+    std::vector<int> idx((size_t)steps * batch), rows;
+    for (int& k : idx) k = pick(rng);
+    int staged = steps > 0 ? stage_tables(L, idx, batch, &rows) : TG_OK;
+    if (staged != TG_OK) return staged;
     for (int s = 0; s < steps; s++) {
-        std::vector<int> idx(batch);
-        for (int& k : idx) k = pick(rng);
-        int rows = 0;
-        int rc = stage_batch(L, idx, &rows);
-        if (rc == TG_OK) rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows);
-        if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows, &losses[s]);
+        stage_batch(L, s, batch, rows[s]);
+        int rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows[s]);
+        if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows[s], L->loss.p + s);
         if (rc != TG_OK) return rc;
         L->adamStep++;
         const float c1 = 1.0f - std::pow(b1, (float)L->adamStep), c2 = 1.0f - std::pow(b2, (float)L->adamStep);
@@ -534,6 +551,7 @@ int tg_learner_train(tg_learner* L, int32_t steps, int32_t batch, float lr, uint
     }
     const int rc = check_status(L, "tg_learner_train");
     if (rc != TG_OK) return rc;
+    if (steps > 0) LCK(cudaMemcpy(losses.data(), L->loss.p, sizeof(float) * steps, cudaMemcpyDeviceToHost));
     if (mean_loss) {
         const int tail = std::max(1, steps / 10);
         double acc = 0.0;

@@ -12,6 +12,7 @@
 // 32 TMEM lanes (rows) with tcgen05.ld.  Every wait on the mbarrier is
 // bounded: on timeout the kernel sets S_TIMEOUT, waits once more (bounded)
 // for the MMAs in flight, frees its TMEM and returns.
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
@@ -61,6 +62,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
     return false;
 }
 
+// The 16-byte piece i of a chunk as (row, K group): a warp takes eight rows
+// by four groups, 512 contiguous bytes of the staged layout (eight groups of
+// four rows put a warp's pieces on the same banks eightfold) and 64 of each
+// row in global memory
+__device__ __forceinline__ int piece_row(int i) { return (i >> 6) * 8 + (i & 7); }
+__device__ __forceinline__ int piece_group(int i) { return ((i >> 5) & 1) * 4 + ((i >> 3) & 3); }
+
 // byte offset of the 16-byte piece (row r, K group k8) of a staged chunk
 __device__ __forceinline__ int tile_off(int r, int k8) { return (r >> 3) * 1024 + k8 * 128 + (r & 7) * 16; }
 
@@ -93,12 +101,12 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16(const __nv_bfloat16*
     const int nk = K / 64;
     for (int kc = 0; kc < nk; kc++) {
         for (int i = tid; i < 128 * 8; i += kGemmThreads) {
-            const int r = i >> 3, c = i & 7;
+            const int r = piece_row(i), c = piece_group(i);
             const uint4 v = *reinterpret_cast<const uint4*>(A + (size_t)(row0 + r) * K + kc * 64 + c * 8);
             *reinterpret_cast<uint4*>(sA + tile_off(r, c)) = v;
         }
         for (int i = tid; i < N * 8; i += kGemmThreads) {
-            const int r = i >> 3, c = i & 7;
+            const int r = piece_row(i), c = piece_group(i);
             const uint4 v = *reinterpret_cast<const uint4*>(B + (size_t)r * K + kc * 64 + c * 8);
             *reinterpret_cast<uint4*>(sB + tile_off(r, c)) = v;
         }
@@ -157,6 +165,170 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16(const __nv_bfloat16*
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(N));
+}
+
+// The same product for a long K and few rows (a weight gradient: 128 x 64
+// with thousands of rows for its K).  One CTA per 128 x 16 tile, its chunks
+// in a ring of kLongStages slots that TMA fills (128-byte swizzle): one
+// thread waits for a slot, issues its MMAs, commits them to the slot's
+// mbarrier and refills the slot of the step before once its MMAs are done.
+// The products are added in the order of k_gemm_bf16, so the result is the
+// same to the bit.  There each chunk's load, MMAs and wait followed one
+// another: 343 us on 4736 rows, most of a training step, against 33
+// here; with cp.async in place of TMA 75, the copies' issue the bound.
+// Sharing K out over CTAs adds in another order, and Adam's first steps carry
+// the last digit of a gradient near zero into the weights.
+constexpr int kLongN = 16, kLongStages = 5, kLongSub = 2;  // chunks of 64 per slot
+constexpr int kLongSubBytes = 16384 + kLongN * 128;
+constexpr int kLongStageBytes = kLongSub * kLongSubBytes;
+constexpr int kLongSmem = kLongStages * kLongStageBytes + 1024;  // slots start on 1024 bytes
+
+// shared-memory matrix descriptor of a K-major tile with the 128-byte
+// swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>(1) << 16;
+    d |= static_cast<uint64_t>((1024u >> 4) & 0x3FFFu) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
+            "r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
+}
+
+__global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_long(const __grid_constant__ CUtensorMap mapA,
+                                                                 const __grid_constant__ CUtensorMap mapB,
+                                                                 float* __restrict__ C, int N, int K, int* status) {
+    extern __shared__ unsigned char smemRaw[];
+    __shared__ uint64_t full[kLongStages], done[kLongStages];
+    __shared__ uint32_t tmemSlot;
+    __shared__ int good;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int row0 = blockIdx.x * 128, col0 = blockIdx.y * kLongN;
+    const uint32_t smem = (smem_u32(smemRaw) + 1023u) & ~1023u;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmemSlot)),
+                     "r"(32));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < kLongStages; k++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[k])), "r"(1));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&done[k])), "r"(1));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tmemSlot;
+    const int chunks = K / 64, steps = (chunks + kLongSub - 1) / kLongSub;
+    if (tid == 0) {
+        int loaded = 0;  // steps whose copies have been issued
+        auto load = [&] {
+            if (loaded >= steps) return;
+            const int slot = loaded % kLongStages;
+            const int subs = min(kLongSub, chunks - loaded * kLongSub);
+            const uint32_t mb = smem_u32(&full[slot]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(subs * kLongSubBytes)
+                         : "memory");
+            for (int sub = 0; sub < subs; sub++) {
+                const uint32_t at = smem + (uint32_t)(slot * kLongStageBytes + sub * kLongSubBytes);
+                const int x = (loaded * kLongSub + sub) * 64;
+                tma_load(at, &mapA, x, row0, mb);
+                tma_load(at + 16384, &mapB, x, col0, mb);
+            }
+            loaded++;
+        };
+        for (int k = 0; k < kLongStages - 1; k++) load();
+        bool ok = true;
+        int issued = 0;
+        for (int kc = 0; kc < steps; kc++) {
+            const int slot = kc % kLongStages;
+            ok = mbar_wait(smem_u32(&full[slot]), (kc / kLongStages) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const int mmas = 4 * min(kLongSub, chunks - kc * kLongSub);
+            for (int ks = 0; ks < mmas; ks++) {
+                const uint32_t at = smem + (uint32_t)(slot * kLongStageBytes + (ks >> 2) * kLongSubBytes + (ks & 3) * 32);
+                const uint64_t ad = umma_desc_sw128(at), bd = umma_desc_sw128(at + 16384);
+                const uint32_t accumulate = (kc > 0 || ks > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                    "l"(ad), "l"(bd), "r"(idesc_bf16(kLongN)), "r"(accumulate));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&done[slot]))
+                         : "memory");
+            issued++;
+            if (kc > 0) {
+                ok = mbar_wait(smem_u32(&done[(kc - 1) % kLongStages]), ((kc - 1) / kLongStages) & 1);
+                if (!ok) break;
+            }
+            load();
+        }
+        // the last MMAs (they complete in order), and after a time-out the
+        // copies still in flight
+        if (issued > 0)
+            ok = mbar_wait(smem_u32(&done[(issued - 1) % kLongStages]), ((issued - 1) / kLongStages) & 1) && ok;
+        for (int k = issued; k < loaded; k++) mbar_wait(smem_u32(&full[k % kLongStages]), (k / kLongStages) & 1);
+        if (!ok) atomicOr(status, S_TIMEOUT);
+        good = ok ? 1 : 0;
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (good) {
+        const int r = row0 + warp * 32 + (tid & 31);
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(tmem + (static_cast<uint32_t>(warp * 32) << 16)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float4* out = reinterpret_cast<float4*>(C + (size_t)r * N + col0);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            out[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                 __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32));
+}
+
+// Tensor map of a row-major BF16 matrix of `rows` rows of K values: boxes of
+// 64 values by boxRows rows, 128-byte swizzle (K a multiple of 64, so a box
+// starts on 128 bytes and never leaves its rows)
+cudaError_t bf16_map(CUtensorMap* map, const void* p, int rows, int K, int boxRows) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {  // initialised once, also under concurrent host threads
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return reinterpret_cast<Encode>(fn);
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)boxRows}, step[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, step,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------------
@@ -321,19 +493,57 @@ __global__ void k_ball_features(DevMesh m, int site, int hops, int D, const int3
     if (phiStart) phiStart[t] = m.phi64[g];
 }
 
+// A tile of kTileRows rows, kept by column so that its transposed copy goes
+// out in runs of rows: the kernels that write an activation both ways are a
+// block per tile, a thread per feature of every fourth row (written straight
+// to a column-major array, each value went to a sector of its own).
+constexpr int kTileRows = 32, kTileThreads = 512, kConcatThreads = 1024;
+template <int kCols>
+struct RowTile {
+    __nv_bfloat16 v[kCols][kTileRows + 2];
+    // out[f * npad + row0 ..] for every column f; npad is a multiple of 128
+    __device__ __forceinline__ void store_transposed(__nv_bfloat16* out, int npad, int row0) const {
+        for (int e = threadIdx.x; e < kCols * (kTileRows / 8); e += blockDim.x) {
+            const int f = e / (kTileRows / 8), r = (e % (kTileRows / 8)) * 8;
+            uint4 w;
+            uint32_t* p = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+            for (int k = 0; k < 4; k++) p[k] = *reinterpret_cast<const uint32_t*>(&v[f][r + 2 * k]);
+            *reinterpret_cast<uint4*>(out + (size_t)f * npad + row0 + r) = w;
+        }
+    }
+};
+// Sum over the block's rows of a thread's value for feature threadIdx.x % 64
+// into out[feature], one atomic per feature
+__device__ __forceinline__ void feature_sum(float s, float* out) {
+    __shared__ float part[kTileThreads];
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kTileThreads / 64; k++) sum += part[threadIdx.x + 64 * k];
+        if (sum != 0.0f) atomicAdd(&out[threadIdx.x], sum);
+    }
+    __syncthreads();
+}
+
 // BF16 input block: features in columns 0..15, zeros to 128; also the
 // transposed copy (column-major) for the weight gradient
 // nDev (may be null): the graph's row count on the device, which caps n
-__global__ void k_input_bf16(const float* X, int n, const int32_t* nDev, int npad, __nv_bfloat16* Z,
-                             __nv_bfloat16* ZT) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npad * kCat) return;
+__global__ void __launch_bounds__(kTileThreads) k_input_bf16(const float* X, int n, const int32_t* nDev, int npad,
+                                                             __nv_bfloat16* Z, __nv_bfloat16* ZT) {
+    __shared__ RowTile<kCat> tile;
+    const int row0 = blockIdx.x * kTileRows;
     if (nDev && *nDev < n) n = *nDev;
-    const int i = t / kCat, f = t % kCat;
-    const float v = (i < n && f < kFeat) ? X[(size_t)i * kFeat + f] : 0.0f;
-    const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    Z[t] = b;
-    ZT[(size_t)f * npad + i] = b;
+    for (int e = threadIdx.x; e < kTileRows * kCat; e += kTileThreads) {
+        const int r = e / kCat, f = e % kCat, i = row0 + r;
+        const __nv_bfloat16 b = __float2bfloat16_rn((i < n && f < kFeat) ? X[(size_t)i * kFeat + f] : 0.0f);
+        Z[(size_t)i * kCat + f] = b;
+        tile.v[f][r] = b;
+    }
+    __syncthreads();
+    tile.store_transposed(ZT, npad, row0);
 }
 
 // u = C + b; h = hPrev + relu(u) (hPrev may be null)
@@ -346,26 +556,53 @@ __global__ void k_bias_act(const float* C, const float* b, const float* hPrev, f
 }
 
 // z = [h, A h] in BF16 (row-major and transposed)
-__global__ void k_message_concat(const float* h, const int32_t* ellCol, const float* ellW, int D, int n,
-                                 const int32_t* nDev, int npad, __nv_bfloat16* Z, __nv_bfloat16* ZT) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npad * kHid) return;
+__global__ void __launch_bounds__(kConcatThreads) k_message_concat(const float* h, const int32_t* ellCol,
+                                                                   const float* ellW, int D, int n,
+                                                                   const int32_t* nDev, int npad, __nv_bfloat16* Z,
+                                                                   __nv_bfloat16* ZT) {
+    __shared__ RowTile<kCat> tile;
+    const int row0 = blockIdx.x * kTileRows;
+    const int f = threadIdx.x % kHid;
     if (nDev && *nDev < n) n = *nDev;
-    const int i = t / kHid, f = t % kHid;
-    float hv = 0.0f, mv = 0.0f;
-    if (i < n) {
-        hv = h[t];
-        for (int k = 0; k < D; k++) {
-            const int j = ellCol[(size_t)i * D + k];
-            if (j < 0) break;
-            mv += ellW[(size_t)i * D + k] * h[(size_t)j * kHid + f];
+    for (int r = threadIdx.x / kHid; r < kTileRows; r += kConcatThreads / kHid) {
+        const int i = row0 + r;
+        float hv = 0.0f, mv = 0.0f;
+        if (i < n) {
+            hv = h[(size_t)i * kHid + f];
+            // four neighbours' loads in flight (D is a multiple of 4 or its
+            // last ones are taken singly; a row ends at its first -1)
+            int k = 0;
+            bool more = true;
+            for (; more && k + 4 <= D; k += 4) {
+                int j[4];
+                float w[4], v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    j[u] = ellCol[(size_t)i * D + k + u];
+                    w[u] = ellW[(size_t)i * D + k + u];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = j[u] >= 0 ? h[(size_t)j[u] * kHid + f] : 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    more = more && j[u] >= 0;
+                    if (more) mv = fmaf(w[u], v[u], mv);
+                }
+            }
+            for (; more && k < D; k++) {
+                const int j = ellCol[(size_t)i * D + k];
+                if (j < 0) break;
+                mv = fmaf(ellW[(size_t)i * D + k], h[(size_t)j * kHid + f], mv);
+            }
         }
+        const __nv_bfloat16 hb = __float2bfloat16_rn(hv), mbv = __float2bfloat16_rn(mv);
+        Z[(size_t)i * kCat + f] = hb;
+        Z[(size_t)i * kCat + kHid + f] = mbv;
+        tile.v[f][r] = hb;
+        tile.v[kHid + f][r] = mbv;
     }
-    const __nv_bfloat16 hb = __float2bfloat16_rn(hv), mbv = __float2bfloat16_rn(mv);
-    Z[(size_t)i * kCat + f] = hb;
-    Z[(size_t)i * kCat + kHid + f] = mbv;
-    ZT[(size_t)f * npad + i] = hb;
-    ZT[(size_t)(kHid + f) * npad + i] = mbv;
+    __syncthreads();
+    tile.store_transposed(ZT, npad, row0);
 }
 
 __global__ void k_readout(const float* h, const float* w, const float* b, int n, const int32_t* nDev, float* y) {
@@ -391,47 +628,69 @@ __global__ void k_loss(const float* y, const float* tgt, int n, float invCount, 
 }
 
 // gradients of the readout; dh = dy w (zero on padding rows)
-__global__ void k_readout_back(const float* h, const float* dy, const float* w, int n, int npad, float* gw, float* gb,
-                               float* dh) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npad * kHid) return;
-    const int i = t / kHid, f = t % kHid;
-    const float d = i < n ? dy[i] : 0.0f;
-    dh[t] = d * w[f];
-    if (d != 0.0f) {
-        atomicAdd(&gw[f], d * h[t]);
-        if (f == 0) atomicAdd(gb, d);
+__global__ void __launch_bounds__(kTileThreads) k_readout_back(const float* h, const float* dy, const float* w, int n,
+                                                               float* gw, float* gb, float* dh) {
+    const int row0 = blockIdx.x * kTileRows;
+    const int f = threadIdx.x % kHid;
+    float sw = 0.0f, sb = 0.0f;
+    for (int r = threadIdx.x / kHid; r < kTileRows; r += kTileThreads / kHid) {
+        const size_t t = (size_t)(row0 + r) * kHid + f;
+        const float d = row0 + r < n ? dy[row0 + r] : 0.0f;
+        dh[t] = d * w[f];
+        if (d != 0.0f) sw += d * h[t];
+        sb += d;
+    }
+    feature_sum(sw, gw);
+    __shared__ float bias[kHid];  // every feature's thread has summed the same rows
+    if (f == 0) bias[threadIdx.x / kHid] = sb;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float sum = 0.0f;
+        for (int k = 0; k < kTileThreads / kHid; k++) sum += bias[k];
+        if (sum != 0.0f) atomicAdd(gb, sum);
     }
 }
 
 // du = dh * [u > 0] (BF16, row-major and transposed); gb += sum du
-__global__ void k_act_back(const float* dh, const float* u, int npad, __nv_bfloat16* DU, __nv_bfloat16* DUT,
-                           float* gb) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npad * kHid) return;
-    const int i = t / kHid, f = t % kHid;
-    const float d = u[t] > 0.0f ? dh[t] : 0.0f;
-    const __nv_bfloat16 b = __float2bfloat16_rn(d);
-    DU[t] = b;
-    DUT[(size_t)f * npad + i] = b;
-    if (d != 0.0f) atomicAdd(&gb[f], d);
+__global__ void __launch_bounds__(kTileThreads) k_act_back(const float* dh, const float* u, int npad,
+                                                           __nv_bfloat16* DU, __nv_bfloat16* DUT, float* gb) {
+    __shared__ RowTile<kHid> tile;
+    const int row0 = blockIdx.x * kTileRows;
+    const int f = threadIdx.x % kHid;
+    float s = 0.0f;
+    for (int r = threadIdx.x / kHid; r < kTileRows; r += kTileThreads / kHid) {
+        const size_t t = (size_t)(row0 + r) * kHid + f;
+        const float d = u[t] > 0.0f ? dh[t] : 0.0f;
+        const __nv_bfloat16 b = __float2bfloat16_rn(d);
+        DU[t] = b;
+        tile.v[f][r] = b;
+        s += d;
+    }
+    feature_sum(s, gb);
+    tile.store_transposed(DUT, npad, row0);
 }
 
 // dhPrev = dh + dz[:, :64]; the message half flows back along the edges:
 // dhPrev[j] += a_ij dz[i, 64 + f]
 __global__ void k_message_back(const float* dh, const float* dz, const int32_t* ellCol, const float* ellW, int D, int n,
                                int npad, float* dhPrev) {
+    // four features a thread, added as one vector
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npad * kHid) return;
-    const int i = t / kHid, f = t % kHid;
-    atomicAdd(&dhPrev[t], dh[t] + dz[(size_t)i * kCat + f]);
+    if (t >= npad * (kHid / 4)) return;
+    const int i = t / (kHid / 4), f = (t % (kHid / 4)) * 4;
+    const float4 a = *reinterpret_cast<const float4*>(dh + (size_t)i * kHid + f);
+    const float4 z = *reinterpret_cast<const float4*>(dz + (size_t)i * kCat + f);
+    atomicAdd(reinterpret_cast<float4*>(dhPrev + (size_t)i * kHid + f),
+              make_float4(a.x + z.x, a.y + z.y, a.z + z.z, a.w + z.w));
     if (i >= n) return;
-    const float dm = dz[(size_t)i * kCat + kHid + f];
-    if (dm == 0.0f) return;
+    const float4 d = *reinterpret_cast<const float4*>(dz + (size_t)i * kCat + kHid + f);
+    if (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f && d.w == 0.0f) return;
     for (int k = 0; k < D; k++) {
         const int j = ellCol[(size_t)i * D + k];
         if (j < 0) break;
-        atomicAdd(&dhPrev[(size_t)j * kHid + f], ellW[(size_t)i * D + k] * dm);
+        const float w = ellW[(size_t)i * D + k];
+        atomicAdd(reinterpret_cast<float4*>(dhPrev + (size_t)j * kHid + f),
+                  make_float4(w * d.x, w * d.y, w * d.z, w * d.w));
     }
 }
 
@@ -520,10 +779,32 @@ __global__ void k_collect_target(DevMesh m, const int32_t* nodes, const int32_t*
     tgt[t] = (float)((m.phi64[nodes[t]] - phiStart[t]) / (double)scale[0]);
 }
 
-// ELL columns of a sample shifted to its place in a batch
-__global__ void k_shift_cols(int32_t* col, int count, int shift) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count && col[t] >= 0) col[t] += shift;
+// A batch gathered from the samples: sample b of the batch is the rows
+// table[b] .. of the sample store and the rows start[b] .. start[b + 1] of the
+// batch (table: batch offsets, then batch + 1 starts), its ELL columns
+// shifted by its start.  One warp per row.
+__global__ void k_stage_batch(const int64_t* __restrict__ table, int batch, int D, const float* __restrict__ sX,
+                              const float* __restrict__ sW, const int32_t* __restrict__ sCol,
+                              const float* __restrict__ sT, float* bX, float* bW, int32_t* bCol, float* bT) {
+    const int64_t* start = table + batch;
+    const int lane = threadIdx.x & 31;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= start[batch]) return;
+    int lo = 0, hi = batch - 1;  // the last sample that starts at or before row i
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (start[mid] <= i) lo = mid;
+        else hi = mid - 1;
+    }
+    const int64_t o = table[lo] + (i - start[lo]);
+    const int shift = (int)start[lo];
+    if (lane < kFeat) bX[i * kFeat + lane] = sX[o * kFeat + lane];
+    for (int k = lane; k < D; k += 32) {
+        const int c = sCol[o * D + k];
+        bCol[i * D + k] = c >= 0 ? c + shift : c;
+        bW[i * D + k] = sW[o * D + k];
+    }
+    if (lane == 0) bT[i] = sT[o];
 }
 
 inline unsigned nblk(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
@@ -539,13 +820,21 @@ cudaError_t launch_gemm_bf16(const void* A, const void* B, float* C, int M, int 
         cudaError_t r = cudaFuncSetAttribute(k_gemm_bf16<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
         if (r == cudaSuccess)
             r = cudaFuncSetAttribute(k_gemm_bf16<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k_gemm_bf16_long, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem);
         return r;
     });
     if (e != cudaSuccess) return e;
     const auto* a = static_cast<const __nv_bfloat16*>(A);
     const auto* b = static_cast<const __nv_bfloat16*>(B);
     count_launch();
-    if (N == 64)
+    // a K of more chunks than the ring holds, on few row tiles: the ring pays
+    if (K / 64 > kLongStages * kLongSub && M / 128 <= 8) {
+        CUtensorMap mapA, mapB;
+        if ((e = bf16_map(&mapA, A, M, K, 128)) != cudaSuccess) return e;
+        if ((e = bf16_map(&mapB, B, N, K, kLongN)) != cudaSuccess) return e;
+        k_gemm_bf16_long<<<dim3(M / 128, N / kLongN), kGemmThreads, kLongSmem, s>>>(mapA, mapB, C, N, K, status);
+    } else if (N == 64)
         k_gemm_bf16<64><<<M / 128, kGemmThreads, kGemmSmem, s>>>(a, b, C, M, K, status);
     else
         k_gemm_bf16<128><<<M / 128, kGemmThreads, kGemmSmem, s>>>(a, b, C, M, K, status);
@@ -573,8 +862,8 @@ void launch_ball_features(const DevMesh& m, int site, int hops, int D, const int
 }
 void launch_input_bf16(const float* X, int n, int npad, void* Z, void* ZT, cudaStream_t s, const int32_t* nDev) {
     count_launch();
-    k_input_bf16<<<nblk((long long)npad * kCat), 256, 0, s>>>(X, n, nDev, npad, static_cast<__nv_bfloat16*>(Z),
-                                                                static_cast<__nv_bfloat16*>(ZT));
+    k_input_bf16<<<npad / kTileRows, kTileThreads, 0, s>>>(X, n, nDev, npad, static_cast<__nv_bfloat16*>(Z),
+                                                            static_cast<__nv_bfloat16*>(ZT));
 }
 void launch_bias_act(const float* C, const float* b, const float* hPrev, float* u, float* h, int npad,
                      cudaStream_t s) {
@@ -584,9 +873,9 @@ void launch_bias_act(const float* C, const float* b, const float* hPrev, float* 
 void launch_message_concat(const float* h, const int32_t* ellCol, const float* ellW, int D, int n, int npad, void* Z,
                            void* ZT, cudaStream_t s, const int32_t* nDev) {
     count_launch();
-    k_message_concat<<<nblk((long long)npad * kHid), 256, 0, s>>>(h, ellCol, ellW, D, n, nDev, npad,
-                                                                    static_cast<__nv_bfloat16*>(Z),
-                                                                    static_cast<__nv_bfloat16*>(ZT));
+    k_message_concat<<<npad / kTileRows, kConcatThreads, 0, s>>>(h, ellCol, ellW, D, n, nDev, npad,
+                                                                static_cast<__nv_bfloat16*>(Z),
+                                                                static_cast<__nv_bfloat16*>(ZT));
 }
 void launch_readout(const float* h, const float* w, const float* b, int n, float* y, cudaStream_t s,
                     const int32_t* nDev) {
@@ -600,17 +889,17 @@ void launch_loss(const float* y, const float* tgt, int n, float invCount, float*
 void launch_readout_back(const float* h, const float* dy, const float* w, int n, int npad, float* gw, float* gb,
                          float* dh, cudaStream_t s) {
     count_launch();
-    k_readout_back<<<nblk((long long)npad * kHid), 256, 0, s>>>(h, dy, w, n, npad, gw, gb, dh);
+    k_readout_back<<<npad / kTileRows, kTileThreads, 0, s>>>(h, dy, w, n, gw, gb, dh);
 }
 void launch_act_back(const float* dh, const float* u, int npad, void* DU, void* DUT, float* gb, cudaStream_t s) {
     count_launch();
-    k_act_back<<<nblk((long long)npad * kHid), 256, 0, s>>>(dh, u, npad, static_cast<__nv_bfloat16*>(DU),
-                                                              static_cast<__nv_bfloat16*>(DUT), gb);
+    k_act_back<<<npad / kTileRows, kTileThreads, 0, s>>>(dh, u, npad, static_cast<__nv_bfloat16*>(DU),
+                                                          static_cast<__nv_bfloat16*>(DUT), gb);
 }
 void launch_message_back(const float* dh, const float* dz, const int32_t* ellCol, const float* ellW, int D, int n,
                          int npad, float* dhPrev, cudaStream_t s) {
     count_launch();
-    k_message_back<<<nblk((long long)npad * kHid), 256, 0, s>>>(dh, dz, ellCol, ellW, D, n, npad, dhPrev);
+    k_message_back<<<nblk((long long)npad * (kHid / 4)), 256, 0, s>>>(dh, dz, ellCol, ellW, D, n, npad, dhPrev);
 }
 void launch_adam(float* p, const float* g, float* m1, float* m2, int count, float lr, float b1, float b2, float eps,
                  float c1, float c2, cudaStream_t s) {
@@ -645,10 +934,12 @@ void launch_collect_target(const DevMesh& m, const int32_t* nodes, const int32_t
     count_launch();
     k_collect_target<<<nblk(cap), 256, 0, s>>>(m, nodes, count, phiStart, scale, tgt);
 }
-void launch_shift_cols(int32_t* col, int count, int shift, cudaStream_t s) {
-    if (count <= 0 || shift == 0) return;
+void launch_stage_batch(const int64_t* table, int batch, int rows, int D, const float* sX, const float* sW,
+                        const int32_t* sCol, const float* sT, float* bX, float* bW, int32_t* bCol, float* bT,
+                        cudaStream_t s) {
+    if (rows <= 0) return;
     count_launch();
-    k_shift_cols<<<nblk(count), 256, 0, s>>>(col, count, shift);
+    k_stage_batch<<<nblk((long long)rows * 32), 256, 0, s>>>(table, batch, D, sX, sW, sCol, sT, bX, bW, bCol, bT);
 }
 
 }  // namespace tgd
