@@ -2107,9 +2107,10 @@ int tg_surface_normals(tg_handle* h, int32_t count, const int32_t* nodes, float*
     if (count == 0) return TG_OK;
     int rc = stage(h, h->stageF, 3 * (size_t)count);
     if (rc == TG_OK) rc = stage(h, h->stageI, count);
+    if (rc == TG_OK) rc = stage(h, h->stageD, 9 * (size_t)count);
     if (rc != TG_OK) return rc;
     CK(cudaMemcpyAsync(h->stageI.p, nodes, sizeof(int32_t) * count, cudaMemcpyHostToDevice, h->stream));
-    launch_surface_normals(h->dm(), h->stageI.p, count, h->vacuumId, h->stageF.p, h->stream);
+    launch_surface_normals(h->dm(), h->stageI.p, count, h->vacuumId, h->stageD.p, h->stageF.p, h->stream);
     CK(cudaMemcpyAsync(normals, h->stageF.p, sizeof(float) * 3 * count, cudaMemcpyDeviceToHost, h->stream));
     return sync_status(h, "tg_surface_normals");
 }
@@ -2125,11 +2126,16 @@ int tg_surface_cells(tg_handle* h, int32_t mode, float temperature, int32_t capa
     if (rc == TG_ERR_NO_SURFACE) return TG_OK;
     if (rc != TG_OK) return rc;
     std::vector<int32_t> list(h->surfSlots);
-    std::vector<float> score(h->surfSlots);
+    std::vector<float> score(capacity > 0 ? h->surfSlots : 0);
     CK(cudaMemcpyAsync(list.data(), h->surfList.p, sizeof(int32_t) * h->surfSlots, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(score.data(), h->surfScore.p, sizeof(float) * h->surfSlots, cudaMemcpyDeviceToHost, h->stream));
+    if (capacity > 0)
+        CK(cudaMemcpyAsync(score.data(), h->surfScore.p, sizeof(float) * h->surfSlots, cudaMemcpyDeviceToHost, h->stream));
     rc = sync_status(h, "tg_surface_cells");
     if (rc != TG_OK) return rc;
+    if (capacity == 0) {  // the count alone
+        *count = (int32_t)(list.size() - std::count(list.begin(), list.end(), -1));
+        return TG_OK;
+    }
     std::vector<std::pair<int32_t, float>> set;
     set.reserve(h->surfSlots);
     for (int s = 0; s < h->surfSlots; s++)

@@ -2,6 +2,8 @@
 // evaporation-field ratio with its argmax, surface-set maintenance, the
 // cell-flip removal with its in-place coupling update, the coordination
 // rewrite and the local surface normal.
+#include <atomic>
+
 #include "kernels.cuh"
 
 namespace tgd {
@@ -480,16 +482,25 @@ __global__ void k_coordination(DevMesh m, const int8_t* before) {
 // 3-hop surface neighbourhood (smallest-eigenvalue eigenvector of the
 // uncentred scatter matrix of p_node - p_k, find_best_plane,
 // geometry_3d.cpp:1806-1870), oriented towards the vacuum cells of the
-// neighbourhood.  One block; Jacobi eigen-iteration in FP64.
+// neighbourhood.  One block finds the neighbourhood and its sums, one thread
+// iterates on them (Jacobi, FP64).
+// The search is bound by its dependent loads (row bounds, neighbours, hash):
+// eight lanes share a frontier cell's row, so that a hop of a hundred cells is
+// a few rounds of them, and the sums are formed in registers (shared FP64
+// atomics on nine words serialised the block's members).  For a list of cells
+// the iterations are a launch of their own, a thread per cell: in the blocks
+// of the search each was one thread's serial chain with the block's shared
+// memory held, and 16,396 surface cells took 3.9 ms against 0.36 so.
 constexpr int kNHash = 4096;
-__device__ void surface_normal(const DevMesh& m, int node, int vacuumId, float* out) {
+constexpr int kNormalThreads = 256, kNormalLanes = 8;
+// sums[0..5]: the scatter of the surface cells (xx, xy, xz, yy, yz, zz),
+// sums[6..8]: the vacuum cells' offsets; written by the first nine threads
+__device__ void surface_sums(const DevMesh& m, int node, int vacuumId, double* sums) {
     __shared__ int32_t keys[kNHash];
     __shared__ int32_t frontier[kNHash];
     __shared__ int fs, fe, tail;
-    __shared__ double S[6], V[3];
+    __shared__ double part[9][kNormalThreads / 32];
     for (int k = threadIdx.x; k < kNHash; k += blockDim.x) keys[k] = -1;
-    if (threadIdx.x < 6) S[threadIdx.x] = 0.0;
-    if (threadIdx.x < 3) V[threadIdx.x] = 0.0;
     if (threadIdx.x == 0) {
         frontier[0] = node;
         fs = 0;
@@ -499,9 +510,10 @@ __device__ void surface_normal(const DevMesh& m, int node, int vacuumId, float* 
     __syncthreads();
     for (int h = 0; h < 3; h++) {
         const int a = fs, b = fe;
-        for (int f = a + threadIdx.x; f < b; f += blockDim.x) {
+        for (int f = a + threadIdx.x / kNormalLanes; f < b; f += kNormalThreads / kNormalLanes) {
             const int u = frontier[f];
-            for (int q = m.row_ptr[u]; q < m.row_ptr[u + 1]; q++) {
+            const int q1 = m.row_ptr[u + 1];
+            for (int q = m.row_ptr[u] + threadIdx.x % kNormalLanes; q < q1; q += kNormalLanes) {
                 const int v = m.col[q];
                 uint32_t hsh = ((uint32_t)v * 2654435761u) & (kNHash - 1);
                 for (int probe = 0; probe < kNHash; probe++) {
@@ -525,26 +537,43 @@ __device__ void surface_normal(const DevMesh& m, int node, int vacuumId, float* 
     }
     const int members = min(tail, kNHash);
     const double px = m.xyz[3 * node], py = m.xyz[3 * node + 1], pz = m.xyz[3 * node + 2];
+    // sums over the members: the scatter of the surface cells, then the
+    // vacuum cells' offsets
+    double sum[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int f = 1 + threadIdx.x; f < members; f += blockDim.x) {
         const int v = frontier[f];
         if (v == node) continue;
         const double dx = m.xyz[3 * v] - px, dy = m.xyz[3 * v + 1] - py, dz = m.xyz[3 * v + 2] - pz;
         if (m.type[v] == vacuumId) {
-            atomicAdd(&V[0], dx);
-            atomicAdd(&V[1], dy);
-            atomicAdd(&V[2], dz);
+            sum[6] += dx;
+            sum[7] += dy;
+            sum[8] += dz;
         }
         if (m.flags[v] & F_SURFACE) {
-            atomicAdd(&S[0], dx * dx);
-            atomicAdd(&S[1], dx * dy);
-            atomicAdd(&S[2], dx * dz);
-            atomicAdd(&S[3], dy * dy);
-            atomicAdd(&S[4], dy * dz);
-            atomicAdd(&S[5], dz * dz);
+            sum[0] += dx * dx;
+            sum[1] += dx * dy;
+            sum[2] += dx * dz;
+            sum[3] += dy * dy;
+            sum[4] += dy * dz;
+            sum[5] += dz * dz;
         }
     }
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const double w = warp_sum(sum[k]);
+        if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = w;
+    }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x < 9) {
+        double w = 0.0;
+        for (int j = 0; j < kNormalThreads / 32; j++) w += part[threadIdx.x][j];
+        sums[threadIdx.x] = w;
+    }
+}
+
+// The normal from surface_sums' sums
+__device__ void normal_from_sums(const double* S, float* out) {
+    const double* V = S + 6;
     double a[3][3] = {{S[0], S[1], S[2]}, {S[1], S[3], S[4]}, {S[2], S[4], S[5]}};
     double ev[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
     for (int sweep = 0; sweep < 64; sweep++) {
@@ -586,12 +615,21 @@ __device__ void surface_normal(const DevMesh& m, int node, int vacuumId, float* 
 }
 
 __global__ void k_surface_normal(DevMesh m, int node, int vacuumId, float* out) {
-    surface_normal(m, node, vacuumId, out);
+    __shared__ double sums[9];
+    surface_sums(m, node, vacuumId, sums);
+    __syncthreads();
+    if (threadIdx.x == 0) normal_from_sums(sums, out);
 }
 
-// The normals of cells nodes[0..count), one block each.
-__global__ void k_surface_normals(DevMesh m, const int32_t* nodes, int vacuumId, float* out) {
-    surface_normal(m, nodes[blockIdx.x], vacuumId, out + 3 * (size_t)blockIdx.x);
+// The sums of cells nodes[0..count), one block each, then their normals, one
+// thread each
+__global__ void __launch_bounds__(kNormalThreads) k_surface_sums(DevMesh m, const int32_t* nodes, int vacuumId,
+                                                                 double* sums) {
+    surface_sums(m, nodes[blockIdx.x], vacuumId, sums + 9 * (size_t)blockIdx.x);
+}
+__global__ void k_surface_normals(int count, const double* __restrict__ sums, float* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < count) normal_from_sums(sums + 9 * (size_t)t, out + 3 * (size_t)t);
 }
 
 inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
@@ -630,11 +668,20 @@ void launch_update_coordination(const DevMesh& m, int8_t* scratchType, cudaStrea
 }
 void launch_surface_normal(const DevMesh& m, Surface sf, int node, int vacuumId, float* out, cudaStream_t s) {
     (void)sf;
-    { count_launch(); k_surface_normal<<<1, 256, 0, s>>>(m, node, vacuumId, out); }
+    { count_launch(); k_surface_normal<<<1, kNormalThreads, 0, s>>>(m, node, vacuumId, out); }
 }
-void launch_surface_normals(const DevMesh& m, const int32_t* nodes, int count, int vacuumId, float* out,
+void launch_surface_normals(const DevMesh& m, const int32_t* nodes, int count, int vacuumId, double* sums, float* out,
                             cudaStream_t s) {
-    if (count > 0) { count_launch(); k_surface_normals<<<count, 256, 0, s>>>(m, nodes, vacuumId, out); }
+    if (count <= 0) return;
+    static std::atomic<uint64_t> done{0};
+    once_per_device(done, [] {  // the search's hash and list are 32 KB a block: as many blocks as threads allow
+        return cudaFuncSetAttribute(k_surface_sums, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    cudaSharedmemCarveoutMaxShared);
+    });
+    count_launch();
+    k_surface_sums<<<count, kNormalThreads, 0, s>>>(m, nodes, vacuumId, sums);
+    count_launch();
+    k_surface_normals<<<(count + 63) / 64, 64, 0, s>>>(count, sums, out);
 }
 void launch_cell_values(const DevMesh& m, const int32_t* nodes, int count, float* phi, float* field, float* force,
                         cudaStream_t s) {
