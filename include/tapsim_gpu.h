@@ -298,7 +298,7 @@ typedef struct {
 } tg_impact;
 /* Trajectory_3d::init/integrate/extrapolate (trajectory_3d.cpp:99-209,
  * 303-332) with o5_integrator (Cash-Karp, :583-676) and
- * errorRestricted_stepper (:358-425), batched: one ion per thread. */
+ * errorRestricted_stepper (:358-425), batched: one ion per warp. */
 int tg_trace(tg_handle* h, int32_t n_ions, const float* start_xyz, const float* start_vel,
              const float* charge_over_mass, const int32_t* tet_guess, const tg_trace_opts* opts, tg_impact* out);
 /* One phase-space point of a flight, Trajectory_3d::phaseVector
@@ -470,12 +470,13 @@ int64_t tg_launch_count(const tg_handle* h);
  * graph, whose kernels read the iteration index and target from device
  * memory (captured again when the hierarchy or the slots in use change),
  * the host reading rho back between batches of replays; 2 (the default)
- * replays it inside a device-side loop (a while-conditional graph node whose last
- * kernel stops it at the target or the iteration cap), one launch per
- * inner solve, its iteration count read with the solve's next residual;
+ * captures the solve's start with it and replays it inside a device-side
+ * loop (a while-conditional graph node whose last kernel stops it at the
+ * target or the iteration cap), one launch per inner solve, its iteration
+ * count read with the solve's next residual;
  * 0 launches each kernel from the host.  All run the same kernels on the
- * same data; the node-space CG of the Neumann rows replays its iteration
- * in modes 1 and 2. */
+ * same data; the node-space CG of the Neumann rows is one launch in modes 1
+ * and 2 (up to 16384 rows; beyond, replays of one captured iteration). */
 int tg_set_launch_mode(tg_handle* h, int32_t mode);
 /* Times `iters` back-to-back launches of one hot kernel on the handle's
  * stream with CUDA events: 0 = FP32 CG SpMV over the non-Neumann free rows,
