@@ -399,11 +399,28 @@ __global__ void k_vcg64_apply(DevMesh m, VSys v, int slots, int record) {
 // agree to the bit when the row is unchanged.
 __device__ void resid_row(const DevMesh& m, int i, double& r, double& b) {
     double s = 0.0, sb = 0.0;
-    for (int q = m.row_ptr[i]; q < m.row_ptr[i + 1]; q++) {
-        const int j = m.col[q];
-        const double c = __dmul_rn(m.ceff64[q], m.phi64[j]);
-        s = __dadd_rn(s, c);
-        if (m.flags[j] & F_DIRICHLET) sb = __dadd_rn(sb, c);
+    const int q1 = m.row_ptr[i + 1];
+    for (int q = m.row_ptr[i]; q < q1; q += 8) {
+        int j[8];
+        double a[8], p[8];
+        bool fixed[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            j[u] = q + u < q1 ? m.col[q + u] : i;
+            a[u] = q + u < q1 ? m.ceff64[q + u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            p[u] = m.phi64[j[u]];
+            fixed[u] = (m.flags[j[u]] & F_DIRICHLET) != 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (q + u >= q1) break;
+            const double c = __dmul_rn(a[u], p[u]);
+            s = __dadd_rn(s, c);
+            if (fixed[u]) sb = __dadd_rn(sb, c);
+        }
     }
     const double qi = m.q64[i];
     r = __dsub_rn(__dsub_rn(s, __dmul_rn(m.diag64[i], m.phi64[i])), qi);
@@ -455,7 +472,13 @@ __device__ __forceinline__ void vsys_set_row_sum(VSys v, int s) {
     const int base = v.slice_start[s >> 5] + (s & 31);
     const int width = v.slice_width[s >> 5];
     double sum = 0.0;
-    for (int k = 0; k < width; k++) sum += v.val[base + 32 * k];
+    for (int k = 0; k < width; k += 8) {
+        float a[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u] = k + u < width ? v.val[base + 32 * (k + u)] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) sum += a[u];
+    }
     v.g[s] = (float)((double)v.d[s] - sum);
 }
 
@@ -493,29 +516,38 @@ __device__ void vsys_add_row(const DevMesh& m, VSys v, int i) {
     const int base = v.slice_start[slice] + r;
     const int width = v.slice_width[slice];
     const int q0 = m.row_ptr[i], q1 = m.row_ptr[i + 1];
-    // entries of the new row (sequential positions among kept neighbours)
-    if (lane == 0) {
-        int k = 0;
-        for (int q = q0; q < q1; q++) {
-            const int j = m.col[q];
+    // entries of the new row (sequential positions among kept neighbours), a
+    // lane per neighbour
+    int taken = 0;
+    for (int b = q0; b < q1; b += 32) {
+        const int q = b + lane;
+        bool keep = false;
+        int j = 0;
+        if (q < q1) {
+            j = m.col[q];
             const uint8_t fj = m.flags[j];
-            const bool keep = !(fj & F_NEUMANN) && (!(fj & F_DIRICHLET) || m.types[m.type[j]].removable);
+            keep = !(fj & F_NEUMANN) && (!(fj & F_DIRICHLET) || m.types[m.type[j]].removable);
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        const int k = taken + __popc(kept & ((1u << lane) - 1u));
+        if (q < q1) {
             if (!keep || k >= width) {
                 v.vpos[q] = -1;
-                continue;
+            } else {
+                const int sj = v.slot_of[j];
+                v.col[base + 32 * k] = sj >= 0 ? sj : v.capacity;
+                vsys_set_val(v, base + 32 * k, m.ceff32[q], m.ceff64[q]);
+                v.vpos[q] = base + 32 * k;
             }
-            const int sj = v.slot_of[j];
-            v.col[base + 32 * k] = sj >= 0 ? sj : v.capacity;
-            vsys_set_val(v, base + 32 * k, m.ceff32[q], m.ceff64[q]);
-            v.vpos[q] = base + 32 * k;
-            k++;
         }
-        for (; k < width; k++) {
-            v.col[base + 32 * k] = v.capacity;
-            vsys_set_val(v, base + 32 * k, 0.0f, 0.0);
-        }
-        vsys_set_row_sum(v, s);
+        taken += __popc(kept);
     }
+    for (int k = min(taken, width) + lane; k < width; k += 32) {
+        v.col[base + 32 * k] = v.capacity;
+        vsys_set_val(v, base + 32 * k, 0.0f, 0.0);
+    }
+    __syncwarp();
+    if (lane == 0) vsys_set_row_sum(v, s);
     __syncwarp();
     // neighbours that are V rows: their entry for i now points at slot s
     for (int q = q0 + lane; q < q1; q += 32) {
