@@ -70,8 +70,10 @@ __device__ __forceinline__ double sweep_row(const DevMesh& m, const SweepRow& r)
 // does not matter).  A colour of a 307k-cell tip is 15k rows, a microsecond's
 // work: small blocks put it on every SM, and as links of a chain
 // (launch_chain) the colours follow one another without a launch's gap.
-// Separate launches of a thread per row that loaded as it went took 193 us a
-// sweep there, these 48.
+// 25 sweeps and the copy of the potentials took 4.8 ms there with a launch per
+// row list and colour and a thread loading its row as it went, 1.8 so; with
+// the rows staged through shared memory by sixteen lanes each the sweeps
+// alone went from 1.58 to 1.77 ms (835k cells: 2.03 to 3.36).
 constexpr int kSweepBlock = 64;
 __global__ void __launch_bounds__(kSweepBlock) k_sweep64(DevMesh m, const int32_t* __restrict__ rowsV, int countV,
                                                          const int32_t* __restrict__ rowsN, int countN,
