@@ -314,7 +314,7 @@ def run_ours(args, rank: int, world: int, dist):
         else run_arm("plain_value", 0, long_run=args.long_events)
     grid, info0, dev_s, t_e2e, phi, clocks = (arm[k] for k in ("grid", "info0", "dev_s", "t_e2e", "phi", "clocks"))
     launches = arm["launches"]
-    # the autotuned schedule of the value arm's hierarchy: per level its rows,
+    # the schedule of the value arm's hierarchy: per level its rows,
     # lanes per CSR row (level 0: the smoothing pass's load depth, 1000+ for
     # the pipelined kernel) and the kept launches' times
     schedule = [{k: (round(v, 4) if isinstance(v, float) else v) for k, v in lv.items()} for lv in grid.amg_schedule()] \

@@ -165,10 +165,11 @@ int tg_solve(tg_handle* h, const tg_solve_opts* opts, tg_solve_info* info);
  * number of coupling loads each lane of the SELL-32 smoothing pass issues
  * ahead of their gathers (4, 8 or 16; 1004 or 1008 for the software-
  * pipelined pass, which loads the next 4 or 8 while it gathers the current
- * ones).  The hierarchy build chooses them
- * one at a time, from a row-length rule, by timing whole V-cycles with
- * each candidate, and keeps a change that takes 3% off the cycle; a_ms /
- * r_ms are the kept kernels' own launch times [ms]. */
+ * ones).  The lanes follow from the matrices' rows and mean row lengths, so
+ * that one specimen's sums are formed in one order; the load depth, which
+ * changes no sum, is the hierarchy build's choice by timing whole V-cycles
+ * (a change is kept when it takes 3% off the cycle).  a_ms / r_ms are the
+ * kernels' own launch times [ms]. */
 int tg_amg_schedule(tg_handle* h, int32_t level, int32_t* rows, int32_t* a_lanes, int32_t* r_lanes, float* a_ms,
                     float* r_ms);
 /* ||r||_2 / ||b||_2 of the current potentials (FP64). */

@@ -380,8 +380,7 @@ float time_launches(F f, int trials, cudaStream_t s, cudaEvent_t e0, cudaEvent_t
 
 }  // namespace
 
-int amg_tune_lanes(AmgDev& g, const VSys& v, int slots, cudaStream_t s, float* aMs, float* rMs, float* fineMs) {
-    static const int kCand[5] = {2, 4, 8, 16, 32};
+int amg_tune(AmgDev& g, const VSys& v, int slots, cudaStream_t s, float* aMs, float* rMs, float* fineMs) {
     constexpr int kTrials = 3;
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess) return -1;
@@ -389,35 +388,28 @@ int amg_tune_lanes(AmgDev& g, const VSys& v, int slots, cudaStream_t s, float* a
         cudaEventDestroy(e0);
         return -1;
     }
-    // The objective is the whole V-cycle as the solve runs it (its output u
-    // and the levels' work vectors are scratch until the solve writes them):
-    // timed alone, a coarse level's matrix stays in L2 and more lanes look
-    // faster, while inside the cycle the fine level's stream has evicted it.
-    // One choice at a time, from the row-length rule's schedule, each kept
-    // only when it takes at least 3% off the cycle.
-    auto cycle = [&] { return time_launches([&] { launch_amg_vcycle(v, slots, g, 0, -1.0, s); }, kTrials, s, e0, e1); };
-    constexpr float kMargin = 0.97f;
-    float best = cycle();
-    auto tryChoice = [&](int* knob, const int* cands, int nc) {
-        const int keep = *knob;
-        int chosen = keep;
-        for (int k = 0; k < nc; k++) {
-            if (cands[k] == keep) continue;
-            *knob = cands[k];
-            const float ms = cycle();
-            if (ms < kMargin * best) {
-                best = ms;
-                chosen = cands[k];
-            }
-        }
-        *knob = chosen;
+    // The objective is the whole V-cycle, chained as the solve runs it (its
+    // output u and the levels' work vectors are scratch until the solve writes
+    // them); a change is kept only when it takes at least 3% off the cycle.
+    auto cycle = [&] {
+        ChainScope chained;
+        return time_launches([&] { launch_amg_vcycle(v, slots, g, 0, -1.0, s); }, kTrials, s, e0, e1);
     };
+    constexpr float kMargin = 0.97f;
     static const int kUnroll[5] = {4, 8, 16, kFinePipe + 4, kFinePipe + 8};
-    tryChoice(&g.fine_unroll, kUnroll, 5);
-    for (int l = 0; l + 1 < g.levels; l++) {
-        tryChoice(&g.lev[l].r_lanes, kCand, 5);
-        if (l + 2 < g.levels) tryChoice(&g.lev[l + 1].a_lanes, kCand, 5);
+    const int keep = g.fine_unroll;
+    int chosen = keep;
+    float best = cycle();
+    for (int u : kUnroll) {
+        if (u == keep) continue;
+        g.fine_unroll = u;
+        const float ms = cycle();
+        if (ms < kMargin * best) {
+            best = ms;
+            chosen = u;
+        }
     }
+    g.fine_unroll = chosen;
     // the kept kernels' own times, for the record
     if (fineMs) {
         const int slices = (slots + 31) / 32;

@@ -153,8 +153,8 @@ struct tg_handle {
     DBuf<float> vVal, vVec;  // vVec: d, x, r, u, w, p, sv, hist, each capacity+1
     DBuf<__nv_bfloat16> vVal16;  // vVal rounded to bf16 (multigrid smoothing pass)
     DBuf<float> vG;              // row sums of the V rows (capacity+1)
-    // timings [ms] of the tuned lane groups of each level's operator and
-    // restriction (amg_tune_lanes), 0 where a level has none
+    // launch times [ms] of each level's operator and restriction (amg_tune),
+    // 0 where a level has none
     float amgTunedA[tgd::kAmgMaxLevels] = {}, amgTunedR[tgd::kAmgMaxLevels] = {};
     float amgTunedFine = 0.0f;  // and of the level-0 pass
     // FP64 inner iterations: couplings at the SELL positions and the vectors
@@ -1489,14 +1489,24 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
     // the DBuf vectors must not reallocate while pointers into them are live
     h->amgI.reserve(8 * H.levels.size() + 4);
     h->amgF.reserve(8 * H.levels.size() + 4);
-    // lanes per CSR row: the power of two nearest a quarter of the mean row
-    // length, so that a lane's entries take about one round of loads
-    auto lanes = [](const tg_host::AmgCsr& M) {
+    // Lanes per CSR row, by a rule on the hierarchy alone: a row's sum is
+    // formed in another order with other lanes, so lanes picked by their times
+    // gave one specimen several sets of last digits, which a flight's last
+    // point turns into 1e-3 of a voltage.  The power of two nearest a quarter
+    // of the mean row length takes a row in about one round of loads (four per
+    // lane); where the launch is bound by its rounds and not by its bytes, a
+    // row is taken in one round (the restriction of the V rows up to 10,000
+    // rows; operators up to 7,000 rows, under V systems whose passes leave
+    // little of them in L2).  These are the lanes that timed trials of the
+    // V-cycle picked most often on 54 specimens of 23k to 835k cells, ten or
+    // twelve times each; on the 7.3M-cell one they are what the trials picked.
+    auto lanes = [](const tg_host::AmgCsr& M, bool oneRound) {
         const double per = M.rows > 0 ? (double)M.val.size() / M.rows / 4.0 : 1.0;
         int L = 2;
-        while (L < 32 && per > L * 1.4142135623730951) L *= 2;
+        while (L < 32 && per > L * (oneRound ? 1.0 : 1.4142135623730951)) L *= 2;
         return L;
     };
+    constexpr int kRoundRowsR = 10000, kRoundRowsA = 7000, kRoundSlots = 25000;
     tgd::AmgDev g{};
     g.levels = (int)H.levels.size();
     for (int l = 0; l < g.levels; l++) {
@@ -1507,7 +1517,7 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
             D.a_ptr = upI(L.A.ptr);
             D.a_col = upI(L.A.col);
             D.a_val = upF(L.A.val);
-            D.a_lanes = lanes(L.A);
+            D.a_lanes = lanes(L.A, slots > kRoundSlots && L.A.rows <= kRoundRowsA);
             std::vector<double> diag(L.A.rows, 1.0);
             for (int i = 0; i < L.A.rows; i++)
                 for (int q = L.A.ptr[i]; q < L.A.ptr[i + 1]; q++)
@@ -1525,7 +1535,7 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
             D.r_ptr = upI(L.R.ptr);
             D.r_col = upI(L.R.col);
             D.r_val = upF(L.R.val);
-            D.r_lanes = lanes(L.R);
+            D.r_lanes = lanes(L.R, l == 0 && L.R.rows <= kRoundRowsR);
         }
     }
     g.y0 = vec((size_t)h->vCapacity + 1);
@@ -1535,10 +1545,10 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
         h->amg_release();
         return cuda_check(h, e, "multigrid upload");
     }
-    // the coarse levels' lane groups from timed trials on this hierarchy
+    // the level-0 pass's load depth, which changes no sum, from timed trials
     for (int l = 0; l < tgd::kAmgMaxLevels; l++) h->amgTunedA[l] = h->amgTunedR[l] = 0.0f;
     g.fine_unroll = 8;
-    if (amg_tune_lanes(g, h->vs(), slots, h->stream, h->amgTunedA, h->amgTunedR, &h->amgTunedFine) != 0) {
+    if (amg_tune(g, h->vs(), slots, h->stream, h->amgTunedA, h->amgTunedR, &h->amgTunedFine) != 0) {
         h->amg_release();
         return cuda_check(h, cudaGetLastError(), "multigrid schedule tuning");
     }

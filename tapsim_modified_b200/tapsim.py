@@ -250,8 +250,8 @@ class Grid:
         N.check(N.lib().tg_set_launch_mode(self._h, int(mode)), self._h)
 
     def amg_schedule(self) -> list[dict]:
-        """Per multigrid level: rows and the tuned lanes per CSR row of its
-        operator and restriction with their launch times (tg_amg_schedule)."""
+        """Per multigrid level: rows and the lanes per CSR row of its operator
+        and restriction with their launch times (tg_amg_schedule)."""
         out = []
         level = 0
         while True:
