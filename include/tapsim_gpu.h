@@ -117,7 +117,8 @@ int tg_local_relax(tg_handle* h, int32_t node, int32_t shell, double threshold, 
 typedef struct {
     double rel_tol;           /* e.g. 1e-8 */
     int32_t max_outer;        /* FP64 defect-correction steps */
-    int32_t max_inner;        /* inner iterations per step */
+    int32_t max_inner;        /* inner iterations per step, >= 0 (at 0, the looped multigrid solve of
+                                 launch mode 2 still takes one) */
     double inner_rtol;        /* inner relative reduction per step */
     /* Start of a solve that follows removals from a converged state:
      *   0  the current potentials (the previous event's solution; plain),

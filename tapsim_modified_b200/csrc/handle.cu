@@ -1576,7 +1576,9 @@ static int amg_setup(tg_handle* h, double* seconds) {
 // fp64: the FP64 iterations (multigrid only), their right-hand side taken
 // from the kept FP64 residuals by node.
 static int run_vcg(tg_handle* h, double rtol, int maxIter, bool amg, int* itersOut, bool fp64 = false) {
-    const size_t need = 4 * (size_t)(maxIter + 2);
+    // the looped solve's body runs once before its cap is tested, and clears
+    // the accumulators of the iteration after it
+    const size_t need = 4 * (size_t)(std::max(maxIter, 1) + 2);
     if (h->vScal.n < need) CK(h->vScal.alloc(need));
     VSys v = h->vs();
     const int slots = h->vActive;
@@ -1676,6 +1678,7 @@ static int run_vcg(tg_handle* h, double rtol, int maxIter, bool amg, int* itersO
 int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
     DeviceScope dev_scope(h);
     if (!h || !o) return fail(h, TG_ERR_ARGUMENT, "tg_solve: null argument");
+    if (o->max_inner < 0) return fail(h, TG_ERR_ARGUMENT, "tg_solve: max_inner below 0");
     if (o->inner_precision < 0 || o->inner_precision > 1)
         return fail(h, TG_ERR_ARGUMENT, "tg_solve: inner_precision 0 (FP32) or 1 (FP64)");
     if (o->inner_precision == 1 && (o->preconditioner != 1 || o->warm_start != 0))
