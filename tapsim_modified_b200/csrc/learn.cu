@@ -226,13 +226,18 @@ int backward(tg_learner* L, const int32_t* col, const float* w, const float* tgt
 
 // The tables of batches of samples (idx: the batches' samples in turn) onto
 // the device, their rows (rowsOut, one per batch), the staging buffers sized
-// for the largest and a zeroed loss for each
+// for the largest and a zeroed loss for each.  A batch that is too large, and
+// those after it, are left out (rowsOut is shorter then).
 int stage_tables(tg_learner* L, const std::vector<int>& idx, int batch, std::vector<int>* rowsOut) {
     const size_t batches = idx.size() / batch, words = 2 * (size_t)batch + 1;
-    std::vector<int64_t> table(batches * words);
+    std::vector<int64_t> table;
     int64_t most = 1;
     rowsOut->clear();
     for (size_t s = 0; s < batches; s++) {
+        int64_t rows = 0;
+        for (int b = 0; b < batch; b++) rows += L->sLen[idx[s * batch + b]];
+        if (rows > (1 << 22)) break;
+        table.resize((s + 1) * words);
         int64_t* off = table.data() + s * words;
         int64_t at = 0;
         for (int b = 0; b < batch; b++) {
@@ -242,16 +247,16 @@ int stage_tables(tg_learner* L, const std::vector<int>& idx, int batch, std::vec
             at += L->sLen[k];
         }
         off[2 * batch] = at;
-        if (at > (1 << 22)) return lfail(L, TG_ERR_ARGUMENT, "learner: batch too large");
         most = std::max(most, at);
         rowsOut->push_back((int)at);
     }
+    if (rowsOut->empty()) return TG_OK;
     const int rc = ensure_rows(L, roundup128((int)most));
     if (rc != TG_OK) return rc;
     if (L->table.n < table.size()) LCK(L->table.alloc(table.size()));
-    if (L->loss.n < batches) LCK(L->loss.alloc(batches));
+    if (L->loss.n < rowsOut->size()) LCK(L->loss.alloc(rowsOut->size()));
     LCK(cudaMemcpyAsync(L->table.p, table.data(), sizeof(int64_t) * table.size(), cudaMemcpyHostToDevice, L->stream));
-    LCK(cudaMemsetAsync(L->loss.p, 0, sizeof(float) * std::max<size_t>(batches, 1), L->stream));
+    LCK(cudaMemsetAsync(L->loss.p, 0, sizeof(float) * rowsOut->size(), L->stream));
     LCK(cudaStreamSynchronize(L->stream));  // the table's host copy ends here
     return TG_OK;
 }
@@ -510,6 +515,7 @@ int tg_learner_gradients(tg_learner* L, int32_t first, int32_t count, float* los
     std::vector<int> rowsOf;
     int rc = stage_tables(L, idx, count, &rowsOf);
     if (rc != TG_OK) return rc;
+    if (rowsOf.empty()) return lfail(L, TG_ERR_ARGUMENT, "learner: batch too large");
     const int rows = rowsOf[0];
     stage_batch(L, 0, count, rows);
     rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows);
@@ -533,25 +539,32 @@ int tg_learner_train(tg_learner* L, int32_t steps, int32_t batch, float lr, uint
     std::uniform_int_distribution<int> pick(first, first + count - 1);
     std::vector<float> losses(steps, 0.0f);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    // every step's samples drawn and their tables sent ahead, the losses read
-    // at the end, so that the steps queue without the host
-    std::vector<int> idx((size_t)steps * batch), rows;
-    for (int& k : idx) k = pick(rng);
-    int staged = steps > 0 ? stage_tables(L, idx, batch, &rows) : TG_OK;
-    if (staged != TG_OK) return staged;
-    for (int s = 0; s < steps; s++) {
-        stage_batch(L, s, batch, rows[s]);
-        int rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows[s]);
-        if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows[s], L->loss.p + s);
+    // the tables of a few steps are drawn and sent ahead, and those steps'
+    // losses read after them, so that the steps queue without the host; a
+    // batch that is too large ends the call at its step
+    constexpr size_t kTableWords = 1 << 16;
+    const int ahead = (int)std::min<size_t>(64, std::max<size_t>(1, kTableWords / (2 * (size_t)batch + 1)));
+    std::vector<int> idx, rows;
+    for (int s0 = 0; s0 < steps; s0 += ahead) {
+        const int n = std::min(ahead, steps - s0);
+        idx.resize((size_t)n * batch);
+        for (int& k : idx) k = pick(rng);
+        int rc = stage_tables(L, idx, batch, &rows);
         if (rc != TG_OK) return rc;
-        L->adamStep++;
-        const float c1 = 1.0f - std::pow(b1, (float)L->adamStep), c2 = 1.0f - std::pow(b2, (float)L->adamStep);
-        launch_adam(L->P.p, L->G.p, L->M1.p, L->M2.p, kParams, lr, b1, b2, eps, c1, c2, L->stream);
-        if ((rc = refresh_bf16(L)) != TG_OK) return rc;
+        for (int s = 0; s < (int)rows.size(); s++) {
+            stage_batch(L, s, batch, rows[s]);
+            rc = forward(L, L->bX.p, L->bCol.p, L->bW.p, rows[s]);
+            if (rc == TG_OK) rc = backward(L, L->bCol.p, L->bW.p, L->bT.p, rows[s], L->loss.p + s);
+            if (rc != TG_OK) return rc;
+            L->adamStep++;
+            const float c1 = 1.0f - std::pow(b1, (float)L->adamStep), c2 = 1.0f - std::pow(b2, (float)L->adamStep);
+            launch_adam(L->P.p, L->G.p, L->M1.p, L->M2.p, kParams, lr, b1, b2, eps, c1, c2, L->stream);
+            if ((rc = refresh_bf16(L)) != TG_OK) return rc;
+        }
+        if ((rc = check_status(L, "tg_learner_train")) != TG_OK) return rc;
+        if ((int)rows.size() < n) return lfail(L, TG_ERR_ARGUMENT, "learner: batch too large");
+        LCK(cudaMemcpy(losses.data() + s0, L->loss.p, sizeof(float) * n, cudaMemcpyDeviceToHost));
     }
-    const int rc = check_status(L, "tg_learner_train");
-    if (rc != TG_OK) return rc;
-    if (steps > 0) LCK(cudaMemcpy(losses.data(), L->loss.p, sizeof(float) * steps, cudaMemcpyDeviceToHost));
     if (mean_loss) {
         const int tail = std::max(1, steps / 10);
         double acc = 0.0;
