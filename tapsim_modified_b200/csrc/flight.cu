@@ -570,14 +570,22 @@ __device__ __forceinline__ bool ck_trial(const DevMesh& m, LaneTet& T, int lane,
         const V3 pa = gather3((double)sx[0]);
         const V3 pb = gather3((double)(sx[1] + wab * dxa));
         const int known = r == 0 ? s0.mode : 0;
-        int Sa = S, ra = 0, rb = 0;
+        int ra = 0, rb = 0;
         bool ina = false, inb = false;
         if (known == 2) {
-            // the walk to b starts from the state's tetrahedron if the warp
-            // still holds it
+            // the walk to b starts from the state's tetrahedron, also after a
+            // trial whose stages ended in others: where b lies on a vertex or
+            // a face, as all-FP32 positions do for many trials, the start
+            // decides which tetrahedron holds it
             const unsigned have = __ballot_sync(0xffffffffu, T.t == s0.tet);
-            if (have) S = __ffs((int)have) - 1;
+            if (have) {
+                S = __ffs((int)have) - 1;
+            } else {
+                S = next = (next + 1) & 31;
+                if (lane == S) load_slot(m, T, s0.tet);
+            }
         }
+        int Sa = S;
         Bary bb = lane_bary(T, pb, &inb);
         if (known == 0) {
             b = lane_bary(T, pa, &ina);
@@ -683,12 +691,13 @@ __device__ __forceinline__ bool error_rule(double relIn, const TraceParams& tp, 
 // the first through a region.  Only a point in none of them walks on
 // (warp_walk), over the lanes' records where the walk crosses them.
 // Measured on the B200: 1000 mixed-precision ions on a 307k-cell tip 15.2 ms
-// with one thread per ion, 6.2 ms so; 4096 FP64 ions on a 500k-cell alloy tip
-// 40.3 and 13.2 ms; the impacts the same to the bit.  About 1300 warp
-// instructions per trial at 5 cycles each (2.2 of them waits on the fixed
-// latency of dependent FP64 arithmetic), instead of 3400.  At 240 registers
-// eight warps fit an SM; 12 or 16 spilled and were slower (8.6 and 10.4
-// against 7.4 ms for 1000 ions).
+// with one thread per ion, 6.1 ms so; 4096 FP64 ions on a 514k-cell alloy tip
+// 40.4 and 10.4 ms (13.2 before the ions beside a coordinate plane started
+// first); impacts and trials of both, and of 7,096 all-FP32 ions, the same to
+// the bit.  About 1300 warp instructions per trial at 5 cycles each (2.2 of
+// them waits on the fixed latency of dependent FP64 arithmetic), instead of
+// 3400.  At 240 registers eight warps fit an SM; in the first version of this
+// kernel (7.4 ms for the 1000 ions) 12 or 16 spilled and took 8.6 and 10.4 ms.
 template <bool kPath, int kPrec>
 __device__ __forceinline__ void trace_ion(const DevMesh& m, V3 x, V3 v, double k, int guessTet, const TraceParams& tp,
                                           unsigned rot, int slot, ImpactOut* out) {
