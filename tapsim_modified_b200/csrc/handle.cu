@@ -102,8 +102,8 @@ struct tg_handle {
     DBuf<int32_t> rowsV, rowsN, allV, allN, segStartD, countVD, countND, countAllD;
     DBuf<int32_t> surfList, surfSlot, surfCount;
     DBuf<float> surfRatio, surfScore;
-    DBuf<float> cgbuf;  // 10 vectors of n floats
-    DBuf<double> scalV, scalN;
+    DBuf<float> cgbuf;  // 5 vectors of n floats
+    DBuf<double> scalN;
     int maxInnerAlloc = 0;
     DBuf<double> acc;
     DBuf<unsigned long long> keys;
@@ -219,15 +219,15 @@ struct tg_handle {
     long long loopStartNodes = 0;        // and of the solve's start before it
     std::vector<uint64_t> iterKey;       // the device state it was captured with
     long long iterNodes = 0;             // kernels in one replay
-    // the same for the node-space CG iterations of either row list (run_cg)
-    cudaGraphExec_t cgExec[2] = {nullptr, nullptr};
-    std::vector<uint64_t> cgKey[2];
-    long long cgNodes[2] = {0, 0};
+    // the same for the node-space CG iterations of the Neumann rows (run_cg)
+    cudaGraphExec_t cgExec = nullptr;
+    std::vector<uint64_t> cgKey;
+    long long cgNodes = 0;
     DBuf<int32_t> cgDone;                // [1] iterations of the last one-launch node-space solve
     DBuf<int32_t> cgIterDev;             // [1] their counter
     DBuf<double> cgTgtDev;               // [2] their targets rel2, abs2
     int lastItersJacobi = 16, lastItersAmg = 4;  // iterations of the last inner solves
-    int lastItersCgV = 16, lastItersCgN = 16;
+    int lastItersCg = 16;
 
     // multigrid preconditioner of the V system (amg.cu): hierarchy built on
     // the host from the V system as it is, uploaded as CSR levels
@@ -374,15 +374,15 @@ struct tg_handle {
         s.capacity = n;
         return s;
     }
-    CGVectors cg(int which) {
+    CGVectors cg() {
         CGVectors v{};
-        float* base = cgbuf.p + (size_t)which * 5 * n;
+        float* base = cgbuf.p;
         v.x = base;
         v.r = base + (size_t)n;
         v.z = base + 2 * (size_t)n;
         v.p = base + 3 * (size_t)n;
         v.ap = base + 4 * (size_t)n;
-        v.scal = which == 0 ? scalV.p : scalN.p;
+        v.scal = scalN.p;
         return v;
     }
 };
@@ -820,8 +820,8 @@ int tg_create(const tg_mesh_desc* d, tg_handle** out) {
     chk(h->surfCount.alloc(1));
     chk(h->surfRatio.alloc(n));
     chk(h->surfScore.alloc(n));
-    chk(h->cgbuf.alloc(10 * (size_t)n));
-    if (e == cudaSuccess) chk(cudaMemset(h->cgbuf.p, 0, 10 * (size_t)n * sizeof(float)));
+    chk(h->cgbuf.alloc(5 * (size_t)n));
+    if (e == cudaSuccess) chk(cudaMemset(h->cgbuf.p, 0, 5 * (size_t)n * sizeof(float)));
     chk(h->acc.alloc(16));
     chk(h->resid.alloc(2 * (size_t)n));
     if (e == cudaSuccess) chk(cudaMemset(h->resid.p, 0, 2 * (size_t)n * sizeof(double)));
@@ -894,7 +894,7 @@ void tg_destroy(tg_handle* h) {
     h->diag32.release(); h->dtypes.release(); h->status.release(); h->rowsV.release(); h->rowsN.release();
     h->allV.release(); h->allN.release(); h->segStartD.release(); h->countVD.release(); h->countND.release();
     h->countAllD.release(); h->surfList.release(); h->surfSlot.release(); h->surfCount.release();
-    h->surfRatio.release(); h->surfScore.release(); h->cgbuf.release(); h->scalV.release(); h->scalN.release(); h->acc.release();
+    h->surfRatio.release(); h->surfScore.release(); h->cgbuf.release(); h->scalN.release(); h->acc.release();
     h->resid.release(); h->rsum.release(); h->resStamp.release(); h->pendingDev.release();
     h->keys.release(); h->result.release(); h->local.release(); h->localCount.release();
     h->localScratch.release(); h->stageI.release(); h->stageD.release(); h->stageF.release();
@@ -909,8 +909,7 @@ void tg_destroy(tg_handle* h) {
     if (h->iterExec) cudaGraphExecDestroy(h->iterExec);
     if (h->loopExec) cudaGraphExecDestroy(h->loopExec);
     h->loopDone.release();
-    for (int w = 0; w < 2; w++)
-        if (h->cgExec[w]) cudaGraphExecDestroy(h->cgExec[w]);
+    if (h->cgExec) cudaGraphExecDestroy(h->cgExec);
     h->cgDone.release();
     h->cgIterDev.release();
     h->cgTgtDev.release();
@@ -1323,9 +1322,9 @@ static int iteration_loop_graph(tg_handle* h, const VSys& v, const VSys& vg) {
     return TG_OK;
 }
 
-// The replayed iteration of the node-space CG on one row list (which: 0 or
-// 1), captured anew when its rows or vectors changed.
-static int cg_iteration_graph(tg_handle* h, int which, const DevMesh& m, const int32_t* rows, int count,
+// The replayed iteration of the node-space CG on the Neumann rows, captured
+// anew when its rows or vectors changed.
+static int cg_iteration_graph(tg_handle* h, const DevMesh& m, const int32_t* rows, int count,
                               const CGVectors& vg) {
     std::vector<uint64_t> key;
     for (const void* q : {(const void*)m.row_ptr, (const void*)m.col, (const void*)m.ceff32, (const void*)m.diag32,
@@ -1334,30 +1333,30 @@ static int cg_iteration_graph(tg_handle* h, int which, const DevMesh& m, const i
                           (const void*)vg.tgt})
         key.push_back((uint64_t)(uintptr_t)q);
     key.push_back((uint64_t)count);
-    if (h->cgExec[which] && key == h->cgKey[which]) return TG_OK;
+    if (h->cgExec && key == h->cgKey) return TG_OK;
     const cudaError_t e = capture_graph(
         h,
         [&](cudaStream_t cs) {
             launch_cg_iter(m, rows, count, vg, 0, -1.0, -1.0, cs);
             launch_cg_replay_step(h->cgIterDev.p, cs);
         },
-        &h->cgExec[which], &h->cgNodes[which]);
+        &h->cgExec, &h->cgNodes);
     if (e != cudaSuccess) return cuda_check(h, e, "tg_solve: node-space CG iteration graph");
-    h->cgKey[which].swap(key);
+    h->cgKey.swap(key);
     return TG_OK;
 }
 
 extern "C" {
 
-static int run_cg(tg_handle* h, int which, const int32_t* rows, int count, double rtol, int maxIter, int* itersOut,
+static int run_cg(tg_handle* h, const int32_t* rows, int count, double rtol, int maxIter, int* itersOut,
                   double absTarget2 = 0.0) {
     DevMesh m = h->dm();
-    CGVectors v = h->cg(which);
-    DBuf<double>& scal = which == 0 ? h->scalV : h->scalN;
+    CGVectors v = h->cg();
+    DBuf<double>& scal = h->scalN;
     const size_t need = 3 * (size_t)(maxIter + 2);
     if (scal.n < need) {
         CK(scal.alloc(need));
-        v = h->cg(which);
+        v = h->cg();
     }
     CK(cudaMemsetAsync(scal.p, 0, sizeof(double) * need, h->stream));
     launch_cg_init(m, rows, count, v, h->stream);
@@ -1373,14 +1372,14 @@ static int run_cg(tg_handle* h, int which, const int32_t* rows, int count, doubl
         CGVectors vg = v;
         vg.iter = h->cgIterDev.p;
         vg.tgt = h->cgTgtDev.p;
-        const int rc = cg_iteration_graph(h, which, m, rows, count, vg);
+        const int rc = cg_iteration_graph(h, m, rows, count, vg);
         if (rc != TG_OK) return rc;
         launch_cg_replay_begin(h->cgIterDev.p, h->cgTgtDev.p, rel2, absTarget2, h->stream);
     }
     int it = 0;
     // iterations queued before the first read: one more than the last solve
     // of this system took, then small batches
-    int& last = which == 0 ? h->lastItersCgV : h->lastItersCgN;
+    int& last = h->lastItersCg;
     int batch = std::min(16, std::max(2, last + 1));
     double sb[3 * 16], s0[3];
     while (it < maxIter) {
@@ -1388,8 +1387,8 @@ static int run_cg(tg_handle* h, int which, const int32_t* rows, int count, doubl
         const int end = std::min(maxIter, it + batch);
         for (; it < end; it++) {
             if (replay) {
-                CK(cudaGraphLaunch(h->cgExec[which], h->stream));
-                g_launches.fetch_add(h->cgNodes[which], std::memory_order_relaxed);
+                CK(cudaGraphLaunch(h->cgExec, h->stream));
+                g_launches.fetch_add(h->cgNodes, std::memory_order_relaxed);
                 continue;
             }
             launch_cg_iter(m, rows, count, v, it, rel2, absTarget2, h->stream);
@@ -1689,7 +1688,7 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
     // or from the kept values) and holds until the next removal
     bool needB = !h->bnormValid;
     VSys vsys = h->vs();
-    CGVectors vN = h->cg(1);
+    CGVectors vN = h->cg();
     tg_solve_info inf{};
     double rel = 0.0;
     // a solve right after removals from a converged state records its
@@ -1870,7 +1869,7 @@ int tg_solve(tg_handle* h, const tg_solve_opts* o, tg_solve_info* info) {
                                    h->stream));
             } else {
                 launch_vcg_couple_neumann(m, vsys, h->allN.p, h->countAllN, vN.r, h->stream, fp64);
-                rc = run_cg(h, 1, h->allN.p, h->countAllN, rtol, o->max_inner, &itN, floor2);
+                rc = run_cg(h, h->allN.p, h->countAllN, rtol, o->max_inner, &itN, floor2);
                 if (rc != TG_OK) return rc;
             }
         }

@@ -271,11 +271,6 @@ void launch_cg_iter(const DevMesh& m, const int32_t* rows, int count, CGVectors 
 constexpr int kCgSolveRows = 16384;
 cudaError_t launch_cg_solve(const DevMesh& m, const int32_t* rows, int count, CGVectors v, const VSys& vs, bool fromX64,
                             double rel2, double abs2, int maxIter, int32_t* iters, cudaStream_t s);
-// the SpMV kernel of one CG iteration on its own (timing hook)
-void launch_cg_spmv_only(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s);
-// rhs_N += sum over non-Neumann free neighbours c_ij x_j (coupling of the
-// Neumann rows to the correction found for the non-Neumann rows)
-void launch_add_coupled(const DevMesh& m, const int32_t* rows, int count, const float* xV, float* r, cudaStream_t s);
 // phi64[i] += x[i] for a row list, and clears the CG vectors on those rows
 void launch_apply_correction(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s);
 // coupling rows: diag64/diag32/ceff from c64 and the flags of all nodes

@@ -179,11 +179,9 @@ __global__ void k_cg_init(DevMesh m, const int32_t* __restrict__ rows, int count
 }
 
 // The target of r.r: rel2 times its start value (scal[2]), and at least
-// abs2; an iteration whose r.r (scal[3it+2]) meets it is done (rel2 < 0:
-// never).  Formed on
+// abs2; an iteration whose r.r (scal[3it+2]) meets it is done.  Formed on
 // the device, so that iterations queue before the host has read r.r.
 __device__ __forceinline__ bool cg_met(const double* scal, int it, double rel2, double abs2) {
-    if (rel2 < 0.0) return false;  // never (launch_cg_spmv_only)
     return scal[3 * it + 2] <= fmax(rel2 * scal[2], abs2);
 }
 
@@ -467,15 +465,6 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(DevMesh m, const int32_
     if (cl.block_rank() == 0 && tid == 0) *iters = it;
 }
 
-__global__ void k_add_coupled(DevMesh m, const int32_t* __restrict__ rows, int count, const float* xV, float* r) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int i = rows[t];
-    float s = 0.0f;
-    for (int q = m.row_ptr[i]; q < m.row_ptr[i + 1]; q++) s += m.ceff32[q] * xV[m.col[q]];
-    r[i] += s;
-}
-
 __global__ void k_apply_correction(DevMesh m, const int32_t* __restrict__ rows, int count, CGVectors v) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
@@ -654,12 +643,6 @@ void launch_cg_replay_begin(int32_t* iter, double* tgt, double rel2, double abs2
 void launch_cg_replay_step(int32_t* iter, cudaStream_t s) {
     count_launch();
     k_cg_replay_step<<<1, 1, 0, s>>>(iter);
-}
-void launch_cg_spmv_only(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s) {
-    if (count > 0) { count_launch(); k_cg_spmv<<<blocks(count), kBlock, 0, s>>>(m, rows, count, v, 0, -1.0, -1.0); }
-}
-void launch_add_coupled(const DevMesh& m, const int32_t* rows, int count, const float* xV, float* r, cudaStream_t s) {
-    if (count > 0) { count_launch(); k_add_coupled<<<blocks(count), kBlock, 0, s>>>(m, rows, count, xV, r); }
 }
 void launch_apply_correction(const DevMesh& m, const int32_t* rows, int count, CGVectors v, cudaStream_t s) {
     if (count > 0) { count_launch(); k_apply_correction<<<blocks(count), kBlock, 0, s>>>(m, rows, count, v); }
