@@ -1494,18 +1494,19 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
     // point turns into 1e-3 of a voltage.  The power of two nearest a quarter
     // of the mean row length takes a row in about one round of loads (four per
     // lane); where the launch is bound by its rounds and not by its bytes, a
-    // row is taken in one round (the restriction of the V rows up to 10,000
-    // rows; operators up to 7,000 rows, under V systems whose passes leave
-    // little of them in L2).  These are the lanes that timed trials of the
-    // V-cycle picked most often on 54 specimens of 23k to 835k cells, ten or
-    // twelve times each; on the 7.3M-cell one they are what the trials picked.
+    // row is taken in one round: the restriction of the V rows up to 11,000
+    // rows, and, under V systems whose passes leave little of them in L2, the
+    // level-1 operator and deeper ones up to 7,000 rows.  These are the lanes
+    // that timed trials of the V-cycle picked most often on 76 specimens of
+    // 23k to 835k cells, ten times or more each (per matrix on 67% to 89% of
+    // the grids); on the 7.3M-cell one they are what the trials picked.
     auto lanes = [](const tg_host::AmgCsr& M, bool oneRound) {
         const double per = M.rows > 0 ? (double)M.val.size() / M.rows / 4.0 : 1.0;
         int L = 2;
         while (L < 32 && per > L * (oneRound ? 1.0 : 1.4142135623730951)) L *= 2;
         return L;
     };
-    constexpr int kRoundRowsR = 10000, kRoundRowsA = 7000, kRoundSlots = 25000;
+    constexpr int kRoundRowsR = 11000, kRoundRowsA = 7000, kRoundSlots = 25000;
     tgd::AmgDev g{};
     g.levels = (int)H.levels.size();
     for (int l = 0; l < g.levels; l++) {
@@ -1516,7 +1517,7 @@ static int amg_setup_impl(tg_handle* h, double* seconds) {
             D.a_ptr = upI(L.A.ptr);
             D.a_col = upI(L.A.col);
             D.a_val = upF(L.A.val);
-            D.a_lanes = lanes(L.A, slots > kRoundSlots && L.A.rows <= kRoundRowsA);
+            D.a_lanes = lanes(L.A, slots > kRoundSlots && (l == 1 || L.A.rows <= kRoundRowsA));
             std::vector<double> diag(L.A.rows, 1.0);
             for (int i = 0; i < L.A.rows; i++)
                 for (int q = L.A.ptr[i]; q < L.A.ptr[i + 1]; q++)
@@ -2462,9 +2463,9 @@ static int trace_impl(tg_handle* h, int32_t nIons, const float* start, const flo
     if (ordered) {
         // the step control bounds the error relative to each component, so an
         // ion beside a coordinate plane of the axis takes the shortest steps:
-        // on a 4096-ion launch the ions with |x| or |y| below a tenth of
-        // their radius (an eighth of them) took 830 trials on average and up
-        // to 2277, the others 390 and up to 1430
+        // on a 4096-ion launch the ions whose smaller one of |x| and |y| is
+        // below a tenth of the larger (an eighth of them) took 830 trials on
+        // average and up to 2277, the others 390 and up to 1430
         order.resize(nIons);
         size_t head = 0, tail = nIons;
         for (int32_t k = 0; k < nIons; k++) {
