@@ -251,7 +251,7 @@ int tg_update_coordination(tg_handle* h);
  * nodes NULL: every cell (count = N).  Any output may be NULL. */
 int tg_cell_values(tg_handle* h, int32_t count, const int32_t* nodes, float* phi_out, float* field_out /* [3*count] */,
                    float* force_out /* [3*count] */);
-/* Surface_3d::Table::normal of each listed cell, one block per cell. */
+/* Surface_3d::Table::normal of each listed cell. */
 int tg_surface_normals(tg_handle* h, int32_t count, const int32_t* nodes, float* normals_out /* [3*count] */);
 /* The surface set in ascending index order with the probabilities of
  * METHOD_EVAPORATION_PROBABILITY prob_mode, normalised as
@@ -275,7 +275,9 @@ typedef struct {
     double error_threshold;     /* TRAJECTORY_ERROR_THRESHOLD */
     int32_t max_steps;          /* iteration bound per ion */
     int32_t stepper_limit;      /* trial steps per accepted step */
-    int32_t walk_limit;         /* tetrahedra per point location */
+    int32_t walk_limit;         /* tetrahedra per walk to a point.  From 256 on, a point is first looked for in
+                                   the flight's last 32 tetrahedra; below, every point is walked to from the
+                                   last one's, and a point exactly on a face may get the face's other side */
     int32_t integrator;         /* TRAJECTORY_INTEGRATOR_TYPE: 0 Euler, 1 Cash-Karp (the reference's default) */
     int32_t stepper;            /* TRAJECTORY_STEPPER_TYPE: 0 none, 1 error-restricted (default),
                                    2 geometry-restricted, 3 adaptive (trajectory_3d.cpp:358-532) */
@@ -476,9 +478,11 @@ int64_t tg_launch_count(const tg_handle* h);
  * loop (a while-conditional graph node whose last kernel stops it at the
  * target or the iteration cap), one launch per inner solve, its iteration
  * count read with the solve's next residual;
- * 0 launches each kernel from the host.  All run the same kernels on the
- * same data; the node-space CG of the Neumann rows is one launch in modes 1
- * and 2 (up to 16384 rows; beyond, replays of one captured iteration). */
+ * 0 launches each kernel from the host.  All run the same kernels of the
+ * multigrid solve on the same data; the node-space CG of the Neumann rows is
+ * one launch in modes 1 and 2 (up to 16384 rows; beyond, replays of one
+ * captured iteration), whose sums are formed in another order than mode 0's:
+ * results agree within the solve's tolerance. */
 int tg_set_launch_mode(tg_handle* h, int32_t mode);
 /* Times `iters` back-to-back launches of one hot kernel on the handle's
  * stream with CUDA events: 0 = FP32 CG SpMV over the non-Neumann free rows,

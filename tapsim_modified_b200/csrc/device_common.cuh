@@ -160,8 +160,9 @@ __device__ __forceinline__ void block_max_atomic_u64(unsigned long long v, unsig
 // Launches a kernel of a chain.  While a ChainScope lives on this thread, the
 // launch may overlap the end of the kernel before it in the stream (the
 // kernel calls chain_wait before it reads what the chain writes); otherwise
-// it is a plain launch.  Used in stream capture, where the chain's first
-// kernel follows the capture's start.
+// it is a plain launch.  A chain's first kernel is a plain launch (the sweeps)
+// or follows the start of a capture (the inner solve) or an idle stream (its
+// timed trials).
 inline thread_local bool t_chain = false;
 struct ChainScope {
     ChainScope() { t_chain = true; }

@@ -495,8 +495,9 @@ __global__ void k_ball_features(DevMesh m, int site, int hops, int D, const int3
 
 // A tile of kTileRows rows, kept by column so that its transposed copy goes
 // out in runs of rows: the kernels that write an activation both ways are a
-// block per tile, a thread per feature of every fourth row (written straight
-// to a column-major array, each value went to a sector of its own).
+// block per tile, a thread per feature of every eighth or sixteenth row
+// (written straight to a column-major array, each value went to a sector of
+// its own).
 constexpr int kTileRows = 32, kTileThreads = 512, kConcatThreads = 1024;
 template <int kCols>
 struct RowTile {
